@@ -51,6 +51,14 @@ class RefineInstance(ctypes.Structure):
                 ('r32', c_void_p), ('e32', c_void_p)]
 
 
+class RowsGroup(ctypes.Structure):
+    _fields_ = [('N', c_void_p), ('W', c_void_p), ('offset', c_int64), ('first', c_int64), ('nq', c_int64)]
+
+
+# afsi_b200_p1_rows_*: info words and the group limit (include/afsi_b200.h)
+ROWS_GROUPS, ROWS_SITES, ROWS_PADDED, ROWS_BOX, ROWS_FLAGS = 24, 0, 3, 6, 7
+
+
 # name -> argtypes (restype int32 unless listed in _RESTYPES)
 _SIGNATURES = {
     'afsi_b200_last_error': [],
@@ -87,6 +95,15 @@ _SIGNATURES = {
     'afsi_b200_hash_accumulate': [c_void_p, c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_int64, c_int32,
                                   c_void_p],
     'afsi_b200_hash_csr_scratch_bytes': [c_int64, c_int32],
+    'afsi_b200_p1_rows_cap': [c_int32],
+    'afsi_b200_p1_rows_scratch_bytes': [c_int64] * 4,
+    'afsi_b200_p1_rows_boxes': [c_void_p, c_int64, c_int64, c_void_p] + [c_int64] * 8 + [c_void_p] * 5,
+    'afsi_b200_p1_rows_incidence': [c_void_p, c_int64, c_int64] + [c_void_p] * 9 + [c_int64, c_void_p],
+    'afsi_b200_p1_rows_fill': [c_void_p, c_void_p, c_int64, c_void_p, c_int32, c_void_p, c_void_p, c_int64, c_void_p,
+                               c_void_p] + [c_int64] * 4 + [c_void_p] * 4 + [c_int32, c_void_p],
+    'afsi_b200_p1_rows_pointers': [c_void_p, c_int64, c_void_p, c_void_p, c_int64, c_void_p],
+    'afsi_b200_p1_rows_finish': [c_void_p, c_void_p, c_int64, c_void_p, c_void_p, c_int64, c_int64] +
+                                [c_void_p] * 6 + [c_int64, c_int32, c_void_p],
     'afsi_b200_hash_csr': [c_void_p, c_void_p, c_int64, c_int64, c_int64] + [c_void_p] * 8 + [c_int64, c_int32,
                                                                                              c_void_p],
     'afsi_b200_csr_spmv': [c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_void_p, c_int64, c_void_p, c_int64,
@@ -207,6 +224,7 @@ _RESTYPES = {'afsi_b200_last_error': ctypes.c_char_p, 'afsi_b200_mg_scratch_byte
              'afsi_b200_p1_plan_scratch_bytes': ctypes.c_int64, 'afsi_b200_hash_csr_scratch_bytes': ctypes.c_int64,
              'afsi_b200_pcg_scratch_bytes': ctypes.c_int64, 'afsi_b200_mg_refine_scratch_bytes': ctypes.c_int64,
              'afsi_b200_stokes_partial_blocks': ctypes.c_int64, 'afsi_b200_cache_scratch_bytes': ctypes.c_int64,
+             'afsi_b200_p1_rows_cap': ctypes.c_int64, 'afsi_b200_p1_rows_scratch_bytes': ctypes.c_int64,
              'afsi_b200_det_plan_bytes': ctypes.c_int64, 'afsi_b200_fe_det_spread_bytes': ctypes.c_int64}
 
 

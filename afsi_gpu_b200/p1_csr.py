@@ -8,14 +8,15 @@ Bᵀ_c·coefficient / cell volume and the interpolation right-hand side is
 B_c·u_c; the consistent-mass solve that the reference wraps around them is
 outside this hot path (the caller supplies the solved coefficient).
 
-Per prepare and component: a support-box plan per quadrature group
-(``afsi_b200_p1_component_plan``), the contraction into a SplitMix64 hash
-(``afsi_b200_hash_contract``, the reference's table format and probe rules),
-retry with a doubled table on overflow, and the table-to-CSR conversion of B
-and Bᵀ (``afsi_b200_hash_csr``).  Host reads are batched: one for the site
-counts of every group and component, one for the three overflow flags, one for
-the three entry counts.  Responses are CSR SpMV launches
-(``afsi_b200_csr_spmv``), summed per row in a fixed order.
+Per prepare the operators are formed row by row, one warp per component and
+node over the union box of the node's cells (``afsi_b200_p1_rows_*``), with two
+host reads: the box sizes and the three entry counts.  Stencils that this form
+does not take (``_assemble_rows``) use the reference's hash: a support-box plan
+per quadrature group (``afsi_b200_p1_component_plan``), the contraction into a
+SplitMix64 hash (``afsi_b200_hash_contract``, the reference's table format and
+probe rules), retry with a doubled table on overflow, and the table-to-CSR
+conversion of B and Bᵀ (``afsi_b200_hash_csr``).  Responses are CSR SpMV
+launches (``afsi_b200_csr_spmv``), summed per row in a fixed order.
 
 ``contract`` and ``hash_accumulate`` keep the signatures of
 ``mac/cuda_ib.py:93-112``.
@@ -250,8 +251,92 @@ class P1CSRTransfer:
 
     @torch.no_grad()
     def assemble_stencil(self, stencil):
-        """B_c and Bᵀ_c for c = 0, 1, 2 (``AssembledP1Transfer.assemble_stencil``
-        with the hash assembly and the CUDA contraction)."""
+        """B_c and Bᵀ_c for c = 0, 1, 2 (``AssembledP1Transfer.assemble_stencil``):
+        row by row where that form takes the stencil (``_assemble_rows``), else
+        the reference's hash assembly with the CUDA contraction."""
+        rows = self._assemble_rows(stencil)
+        return self._assemble_hash(stencil) if rows is None else rows
+
+    def _rows_scratch(self, nbytes, device):
+        if self._plan_scratch is None or self._plan_scratch.numel() < nbytes or self._plan_scratch.device != device:
+            self._plan_scratch = torch.empty(int(nbytes), dtype=torch.uint8, device=device)
+        return self._plan_scratch
+
+    def _assemble_rows(self, stencil):
+        """The operators node by node (``csrc/csr_rows.cu``): two host reads, no
+        table, values in a fixed order.  None where the hash form is to be used:
+        tables of another layout or type, more groups than one launch takes, a
+        node id or support out of range (the hash form raises it), a row whose
+        box exceeds shared memory, or rows so much wider than their cells'
+        boxes that the padded rows would outgrow half the cells' entries."""
+        groups, base, phi = stencil.rule.groups, stencil.base, stencil.phi
+        like, dev, lib = groups[0].weights, stencil.base.device, _lib.load()
+        elements, nodes, shape = sum(g.cells.shape[0] for g in groups), self.node_count, self.grid.shape
+        if (getattr(stencil, 'layout', None) != 'shared' or len(groups) > _lib.ROWS_GROUPS or
+                like.dtype not in (torch.float32, torch.float64) or not 0 < elements < 2 ** 29 or
+                not 0 < nodes < 2 ** 31 - 1 or prod(n + 1 for n in shape) >= 2 ** 31 - 1 or
+                max(shape) >= 1 << 20 or phi.data_ptr() % 16 or base.dtype != torch.int64 or
+                any(t.dtype != like.dtype for g in groups for t in (g.values, g.weights)) or phi.dtype != like.dtype or
+                not all(t.is_contiguous() and t.device == dev for g in groups for t in (g.cells, g.values, g.weights)) or
+                not (base.is_contiguous() and phi.is_contiguous() and phi.device == dev)):
+            return None
+        total, s, code = base.shape[1], stream(dev), dtype_code(like.dtype)
+        new = lambda n, dt: torch.empty(n, dtype=dt, device=dev)
+        box, keys, slots_in = new(12 * elements, torch.int32), new(4 * elements, torch.int32), new(4 * elements, torch.int32)
+        info = torch.zeros(8, dtype=torch.int64, device=dev)
+        table = (_lib.RowsGroup * len(groups))()
+        offset = first = 0
+        for k, g in enumerate(groups):
+            table[k] = _lib.RowsGroup(ptr(g.values), ptr(g.weights), offset, first, g.values.shape[0])
+            call('afsi_b200_p1_rows_boxes', ptr(base), total, offset, ptr(g.cells), g.cells.shape[0], g.values.shape[0],
+                 first, elements, nodes, *shape, ptr(box), ptr(keys), ptr(slots_in), ptr(info), s)
+            offset += g.weights.numel()
+            first += g.cells.shape[0]
+        start, slots, node_box = new(nodes + 1, torch.int32), new(4 * elements, torch.int32), new(12 * nodes, torch.int32)
+        volume, row_off = new(3 * nodes, torch.int64), new(3 * nodes, torch.int64)
+        scratch = self._rows_scratch(lib.afsi_b200_p1_rows_scratch_bytes(elements, nodes, 0, 0), dev)
+        call('afsi_b200_p1_rows_incidence', ptr(box), elements, nodes, ptr(keys), ptr(slots_in), ptr(start), ptr(slots),
+             ptr(node_box), ptr(volume), ptr(row_off), ptr(info), ptr(scratch), scratch.numel(), s)
+        counts = info.tolist()
+        sites, padded = counts[_lib.ROWS_SITES:_lib.ROWS_SITES + 3], counts[_lib.ROWS_PADDED:_lib.ROWS_PADDED + 3]
+        cap = counts[_lib.ROWS_BOX]
+        if counts[_lib.ROWS_FLAGS] or not 0 < cap <= lib.afsi_b200_p1_rows_cap(code) or sum(padded) > 2 * sum(sites):
+            return None
+        pcol, pval = new(sum(padded), torch.int32), new(sum(padded), like.dtype)
+        row_counts = volume  # the volumes are used up
+        call('afsi_b200_p1_rows_fill', ptr(base), ptr(phi), total, table, len(groups), ptr(start), ptr(slots), nodes,
+             ptr(node_box), ptr(row_off), *shape, cap, ptr(pcol), ptr(pval), ptr(row_counts), ptr(info), code, s)
+        crows = [new(nodes + 1, torch.int64) for _ in range(3)]
+        for c in range(3):
+            call('afsi_b200_p1_rows_pointers', ptr(row_counts[c * nodes:]), nodes, ptr(crows[c]), ptr(scratch),
+                 scratch.numel(), s)
+        *nnz, flags = torch.stack([crow[-1] for crow in crows] + [info[_lib.ROWS_FLAGS]]).tolist()
+        if sum(nnz) > self.max_entries:
+            raise RuntimeError('assembled IB entry budget exceeded; no hash entries were truncated')
+        if max(nnz) >= 2 ** 31 - 1:
+            return None
+        if flags:
+            raise FloatingPointError('invalid hash IB entries: nonfinite values or out-of-range keys')
+        gather, spread, stats = [], [], []
+        sizes = [prod(self.grid.face_shape(c)) for c in range(3)]
+        scratch = self._rows_scratch(lib.afsi_b200_p1_rows_scratch_bytes(0, 0, max(nnz), max(sizes)), dev)
+        for c, (crow, n, nf) in enumerate(zip(crows, nnz, sizes)):
+            col, val = new(n, torch.int64), new(n, like.dtype)
+            t_crow, t_col, t_val = new(nf + 1, torch.int64), new(n, torch.int64), new(n, like.dtype)
+            call('afsi_b200_p1_rows_finish', ptr(crow), ptr(row_off[c * nodes:]), nodes, ptr(pcol), ptr(pval), n, nf,
+                 ptr(col), ptr(val), ptr(t_crow), ptr(t_col), ptr(t_val), ptr(scratch), scratch.numel(), code, s)
+            gather.append(CSR(crow, col, val, (nodes, nf)))
+            spread.append(CSR(t_crow, t_col, t_val, (nf, nodes)))
+            stats.append(dict(raw_cell_entries=4 * sites[c], nnz=n, hash_capacity=0, hash_attempts=0,
+                              hash_workspace_bytes=0, hash_workspace_allocations=0, hash_workspace_reuses=0,
+                              raw_entries_materialized=False, unique_key_sorts=1, duplicate_merge_sorts=0))
+        self.csr_builds += 1
+        return AssembledStencil(tuple(gather), tuple(spread), stencil.rule,
+                                dict(components=stats, total_nnz=sum(nnz), max_entries=self.max_entries,
+                                     assembly_backend='rows', contraction_backend='cuda',
+                                     builder='b200-node-rows+radix-transpose'))
+
+    def _assemble_hash(self, stencil):
         like = stencil.rule.groups[0].weights
         plans = self._plans(stencil)
         limit = power_of_two(2 * self.max_entries)

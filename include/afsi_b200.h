@@ -200,6 +200,60 @@ int32_t afsi_b200_cached_contract(const int64_t* base, const void* phi, const vo
 int32_t afsi_b200_hash_accumulate(const int64_t* input_keys, const void* input_values, int64_t count,
     int64_t* keys, void* values, int32_t* flag, int64_t capacity, int32_t dtype, afsi_stream_t stream);
 
+/* The same operators without a table (csrc/csr_rows.cu): rows of B formed
+ * node by node over the shared tables (lattice 0 faces, 1 centres), for all
+ * three components, every quadrature group's elements numbered one after the
+ * other.  Results: B and its transpose as afsi_b200_hash_csr gives them, the
+ * values summed in a fixed order.
+ *   boxes      one call per group (elements first .. first + group_elements):
+ *              box (device int32[3 * elements * 4]), keys / slots
+ *              (device [4 * elements]); info (device uint64[8], zeroed before
+ *              the first call);
+ *   incidence  start (nodes + 1), slots (4 * elements), node_box
+ *              (int32[3 * nodes * 4]), volume / row_off (int64[3 * nodes]);
+ *   info       [AFSI_ROWS_SITES + c] box sites of component c's elements,
+ *              [AFSI_ROWS_PADDED + c] padded row entries of component c,
+ *              [AFSI_ROWS_BOX] largest shared-memory box, [AFSI_ROWS_FLAGS] bit 0:
+ *              a node id or a support box out of range (use the table form, which
+ *              reports it), bit 1 (fill): a nonfinite value;
+ *   fill       pcol / pval (all components' padded entries), counts
+ *              (int64[3 * nodes]); box_cap >= info[AFSI_ROWS_BOX], at most
+ *              afsi_b200_p1_rows_cap(dtype);
+ *   pointers   crow (nodes + 1) of one component from its counts;
+ *   finish     one component: col / val (nnz), t_crow (nf + 1), t_col / t_val
+ *              (nnz), row_off and counts at that component's rows.
+ * scratch: afsi_b200_p1_rows_scratch_bytes(elements, nodes, nnz, nf) device
+ * bytes (0 for what a call does not use). */
+#define AFSI_ROWS_GROUPS 24
+#define AFSI_ROWS_SITES 0
+#define AFSI_ROWS_PADDED 3
+#define AFSI_ROWS_BOX 6
+#define AFSI_ROWS_FLAGS 7
+typedef struct {
+    const void* N;   /* (nq, 4) shape values */
+    const void* W;   /* (elements of the group, nq) weights */
+    int64_t offset;  /* first table row */
+    int64_t first;   /* first element */
+    int64_t nq;
+} afsi_rows_group;
+int64_t afsi_b200_p1_rows_cap(int32_t dtype);
+int64_t afsi_b200_p1_rows_scratch_bytes(int64_t elements, int64_t nodes, int64_t nnz, int64_t nf);
+int32_t afsi_b200_p1_rows_boxes(const int64_t* base, int64_t total, int64_t offset, const int64_t* cells,
+    int64_t group_elements, int64_t nq, int64_t first, int64_t elements, int64_t nodes, int64_t nx, int64_t ny,
+    int64_t nz, int32_t* box, uint32_t* keys, int32_t* slots, uint64_t* info, afsi_stream_t stream);
+int32_t afsi_b200_p1_rows_incidence(const int32_t* box, int64_t elements, int64_t nodes, const uint32_t* keys,
+    const int32_t* slots_in, int32_t* start, int32_t* slots, int32_t* node_box, int64_t* volume, int64_t* row_off,
+    uint64_t* info, void* scratch, int64_t scratch_bytes, afsi_stream_t stream);
+int32_t afsi_b200_p1_rows_fill(const int64_t* base, const void* phi, int64_t total, const afsi_rows_group* groups,
+    int32_t group_count, const int32_t* start, const int32_t* slots, int64_t nodes, const int32_t* node_box,
+    const int64_t* row_off, int64_t nx, int64_t ny, int64_t nz, int64_t box_cap, int32_t* pcol, void* pval,
+    int64_t* counts, uint64_t* info, int32_t dtype, afsi_stream_t stream);
+int32_t afsi_b200_p1_rows_pointers(const int64_t* counts, int64_t nodes, int64_t* crow, void* scratch,
+    int64_t scratch_bytes, afsi_stream_t stream);
+int32_t afsi_b200_p1_rows_finish(const int64_t* crow, const int64_t* row_off, int64_t nodes, const int32_t* pcol,
+    const void* pval, int64_t nnz, int64_t nf, int64_t* col, void* val, int64_t* t_crow, int64_t* t_col,
+    void* t_val, void* scratch, int64_t scratch_bytes, int32_t dtype, afsi_stream_t stream);
+
 /* Table -> CSR of B (rows x nf, key = row*nf + col) and of its transpose
  * (finish_component, mac/hash_transfer_assembly.py:105-119): crow (rows+1),
  * col/val (capacity; the first nnz are B's entries, column-sorted rows),
