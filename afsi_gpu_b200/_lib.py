@@ -122,6 +122,12 @@ _SIGNATURES = {
                                  c_void_p, c_int32, c_void_p],
     'afsi_b200_compact_spread': [c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int64, c_int64, c_double,
                                  c_void_p, c_void_p, c_int32, c_void_p],
+    'afsi_b200_compact_gather3': [c_void_p] * 5 + [c_int64] * 4 + [c_void_p, c_void_p, c_int32, c_void_p],
+    'afsi_b200_compact_spread3': [c_void_p] * 3 + [c_int64] * 4 + [c_double] + [c_void_p] * 4 + [c_int32, c_void_p],
+    'afsi_b200_indexed_gather2': [c_void_p, c_void_p, c_int64, c_int64] + [c_void_p] * 4 +
+                                 [c_int64, c_void_p, c_void_p, c_int32, c_void_p],
+    'afsi_b200_indexed_spread2': [c_void_p, c_int64] + [c_void_p] * 4 + [c_int64] * 3 + [c_double] + [c_void_p] * 3 +
+                                 [c_int32, c_void_p],
     'afsi_b200_p2_spread': [c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_void_p, c_void_p,
                             c_int64, c_int64, c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int64, c_double,
                             c_void_p, c_int32, c_void_p],

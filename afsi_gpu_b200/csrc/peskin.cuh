@@ -4,15 +4,15 @@
 
 namespace afsi {
 
-// Clamped two-branch Peskin kernel, afsi_torch/ib.py:57-67.
+// Clamped two-branch Peskin kernel, afsi_torch/ib.py:57-67.  Only the branch
+// that applies is evaluated (one square root): the taps of one offset fall in
+// the same branch for all points but those on a grid line.
 template <class T>
 __device__ __forceinline__ T peskin_clamped(T d) {
     const T r = fabs(d);
-    const T a = r < T(1) ? r : T(1);
-    const T b = r < T(1) ? T(1) : (r < T(2) ? r : T(2));
-    const T inner = (T(3) - T(2) * a + sqrt(T(1) + T(4) * a - T(4) * (a * a))) / T(8);
-    const T outer = (T(5) - T(2) * b - sqrt(T(-7) + T(12) * b - T(4) * (b * b))) / T(8);
-    return r < T(1) ? inner : (r < T(2) ? outer : T(0));
+    if (r < T(1)) return (T(3) - T(2) * r + sqrt(T(1) + T(4) * r - T(4) * (r * r))) / T(8);
+    if (r < T(2)) return (T(5) - T(2) * r - sqrt(T(-7) + T(12) * r - T(4) * (r * r))) / T(8);
+    return T(0);
 }
 
 // Shared-radical weights for f in [0,1), mac/csrc/p2_transfer.cu:36-43.

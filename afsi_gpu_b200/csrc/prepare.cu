@@ -2,7 +2,7 @@
 //
 // One thread per point: the point's coordinates are read once and all of its
 // lattices and axes are produced from registers, so the only HBM traffic is
-// the point read and the table write.  Arithmetic follows the reference
+// the point read and the table write, which goes through shared memory.  Arithmetic follows the reference
 // operation order (library built with --fmad=false, IEEE division and sqrt),
 // which makes the integer bases bit-exact and the weights equal to rounding.
 #include "common.cuh"
@@ -22,6 +22,10 @@ __device__ __forceinline__ void store4<float>(float* dst, const float w[4]) {
     *reinterpret_cast<float4*>(dst) = make_float4(w[0], w[1], w[2], w[3]);
 }
 
+template <class T> struct CompactVec16;
+template <> struct CompactVec16<double> { using type = double2; };
+template <> struct CompactVec16<float> { using type = float4; };
+
 template <class T>
 struct CompactParams {
     T origins[3][3];
@@ -32,39 +36,62 @@ struct CompactParams {
     int form;
 };
 
-template <class T>
-__global__ void __launch_bounds__(256) compact_prepare_kernel(const T* __restrict__ points, int64_t count,
-                                                              CompactParams<T> prm, int64_t* __restrict__ base,
-                                                              T* __restrict__ phi, int32_t* status) {
-    const int64_t p = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (p >= count) return;
-    T x[3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a) x[a] = points[p * 3 + a];
-    bool valid = true;
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        const T s = (x[a] - prm.grid_origin[a]) / prm.spacing[a];
-        valid = valid && isfinite(s) && s >= T(2) && s < prm.limits[a];
-    }
-    if (!valid) flag(status, AFSI_FLAG_SUPPORT);
-    for (int l = 0; l < prm.lattices; ++l) {
+// One thread per point; a block's rows of a lattice (3 bases, 12 weights per
+// point) are staged in shared memory and leave as two contiguous ranges, so the
+// stores are whole lines instead of 8 to 32 bytes per point and axis (400,000
+// points, three lattices, FP64: 57 -> 35 us for 154 MB, 4.4 TB/s).
+constexpr int kCompactThreads = 128;
+
+template <class T, bool Aligned>
+__global__ void __launch_bounds__(kCompactThreads) compact_prepare_kernel(const T* __restrict__ points, int64_t count,
+                                                                          CompactParams<T> prm,
+                                                                          int64_t* __restrict__ base,
+                                                                          T* __restrict__ phi, int32_t* status) {
+    __shared__ __align__(16) T s_phi[kCompactThreads * 12];
+    __shared__ int64_t s_base[kCompactThreads * 3];
+    const int64_t first = int64_t(blockIdx.x) * kCompactThreads;
+    const int n = int(count - first < kCompactThreads ? count - first : kCompactThreads);
+    const int t = threadIdx.x;
+    T x[3] = {T(0), T(0), T(0)};
+    if (t < n) {
+        bool valid = true;
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
-            const T scaled = (x[a] - prm.origins[l][a]) / prm.spacing[a];
-            const T lo = floor(scaled - T(1));
-            const int64_t lower = static_cast<int64_t>(lo);
-            const int64_t row = (l * count + p) * 3 + a;
-            base[row] = lower;
-            T w[4];
-            if (prm.form == AFSI_PHI_RADICAL) {
-                peskin_radical(scaled - T(lower) - T(1), w);
-            } else {
-#pragma unroll
-                for (int k = 0; k < 4; ++k) w[k] = peskin_clamped(scaled - T(lower + k));
-            }
-            store4(phi + row * 4, w);
+            x[a] = points[(first + t) * 3 + a];
+            const T s = (x[a] - prm.grid_origin[a]) / prm.spacing[a];
+            valid = valid && isfinite(s) && s >= T(2) && s < prm.limits[a];
         }
+        if (!valid) flag(status, AFSI_FLAG_SUPPORT);
+    }
+    for (int l = 0; l < prm.lattices; ++l) {
+        if (t < n) {
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                const T scaled = (x[a] - prm.origins[l][a]) / prm.spacing[a];
+                const int64_t lower = static_cast<int64_t>(floor(scaled - T(1)));
+                s_base[t * 3 + a] = lower;
+                T w[4];
+                if (prm.form == AFSI_PHI_RADICAL) {
+                    peskin_radical(scaled - T(lower) - T(1), w);
+                } else {
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) w[k] = peskin_clamped(scaled - T(lower + k));
+                }
+                store4(s_phi + (t * 3 + a) * 4, w);
+            }
+        }
+        __syncthreads();
+        const int64_t row = (l * count + first) * 3;
+        for (int i = t; i < n * 3; i += kCompactThreads) base[row + i] = s_base[i];
+        if constexpr (Aligned) {  // row * 4 values: a multiple of 12, so 16-byte aligned with the table
+            using V = typename CompactVec16<T>::type;
+            V* dst = reinterpret_cast<V*>(phi + row * 4);
+            const V* src = reinterpret_cast<const V*>(s_phi);
+            for (int i = t; i < n * 12 * int(sizeof(T)) / 16; i += kCompactThreads) dst[i] = src[i];
+        } else {
+            for (int i = t; i < n * 12; i += kCompactThreads) phi[row * 4 + i] = s_phi[i];
+        }
+        __syncthreads();
     }
 }
 
@@ -361,8 +388,13 @@ extern "C" int32_t afsi_b200_compact_prepare(const void* points, int64_t count, 
         }
         prm.lattices = lattices;
         prm.form = phi_form;
-        compact_prepare_kernel<T><<<blocks_for(count, 256), 256, 0, stream>>>(
-            static_cast<const T*>(points), count, prm, base, static_cast<T*>(phi), status);
+        const unsigned blocks = blocks_for(count, kCompactThreads);
+        if (reinterpret_cast<uintptr_t>(phi) % 16 == 0)
+            compact_prepare_kernel<T, true><<<blocks, kCompactThreads, 0, stream>>>(
+                static_cast<const T*>(points), count, prm, base, static_cast<T*>(phi), status);
+        else
+            compact_prepare_kernel<T, false><<<blocks, kCompactThreads, 0, stream>>>(
+                static_cast<const T*>(points), count, prm, base, static_cast<T*>(phi), status);
     });
     return launched("compact_prepare");
 }

@@ -14,6 +14,7 @@ Beyond the reference operators this module exposes the binning kernels
 expressions.
 """
 from dataclasses import dataclass
+from math import prod
 import torch
 from . import _lib
 from ._lib import call, ptr, stream, dtype_code
@@ -144,8 +145,33 @@ def indexed_spread(field, indices, weights, size, volume=1.):
     return op_indexed_spread(field.contiguous(), indices.contiguous(), weights.contiguous(), size, float(volume))
 
 
+def _component_tables(grid, values, stencil, like):
+    """(base, phi) of a stencil with one contiguous table per component, for
+    the one-launch transfers; None for any other (lists, views, other types),
+    which takes the per-component operators and their checks."""
+    base, phi = stencil.base, stencil.phi
+    if not (torch.is_tensor(base) and torch.is_tensor(phi) and base.dim() == 3 and base.shape[0] == 3
+            and base.shape[2] == 3 and phi.shape == (*base.shape, 4) and base.dtype == torch.int64
+            and phi.dtype == like.dtype and like.dtype in (torch.float32, torch.float64)
+            and base.is_contiguous() and phi.is_contiguous()
+            and all(t.device == like.device and not t.requires_grad for t in (base, phi, *values))
+            and all(grid.face_shape(c) == tuple(n + (a == c) for a, n in enumerate(grid.shape)) for c in range(3))
+            and min(grid.shape) > 0):
+        return None
+    return base, phi
+
+
 def compact_gather(grid, velocity, stencil):
     require_cuda(velocity[0])
+    tables = _component_tables(grid, velocity, stencil, velocity[0]) if len(velocity) == 3 else None
+    if tables is not None and all(u.dtype == velocity[0].dtype and u.numel() == prod(grid.face_shape(c))
+                                  for c, u in enumerate(velocity)):
+        base, phi = tables
+        u = [u.contiguous() for u in velocity]
+        out = torch.empty((base.shape[1], 3), device=base.device, dtype=phi.dtype)
+        call('afsi_b200_compact_gather3', *(ptr(t) for t in u), ptr(base), ptr(phi), base.shape[1], *grid.shape,
+             ptr(out), ptr(_lib.status_word(base.device)), dtype_code(phi.dtype), stream(base.device))
+        return out
     return torch.stack([op_compact_gather(u.contiguous().view(-1), stencil.base[c].contiguous(),
                                           stencil.phi[c].contiguous(), *grid.face_shape(c))
                         for c, u in enumerate(velocity)], -1)
@@ -153,6 +179,15 @@ def compact_gather(grid, velocity, stencil):
 
 def compact_spread(grid, force, stencil):
     require_cuda(force)
+    tables = _component_tables(grid, (force,), stencil, force)
+    if tables is not None and force.shape == (tables[0].shape[1], 3) and grid.volume > 0:
+        base, phi = tables
+        force = force.contiguous()
+        fields = tuple(torch.empty(grid.face_shape(c), device=force.device, dtype=force.dtype) for c in range(3))
+        call('afsi_b200_compact_spread3', ptr(force), ptr(base), ptr(phi), base.shape[1], *grid.shape,
+             float(grid.volume), *(ptr(f) for f in fields), ptr(_lib.status_word(force.device)),
+             dtype_code(force.dtype), stream(force.device))
+        return fields
     return tuple(op_compact_spread(force[:, c].contiguous(), stencil.base[c].contiguous(),
                                    stencil.phi[c].contiguous(), *grid.face_shape(c),
                                    float(grid.volume)).view(grid.face_shape(c)) for c in range(3))
@@ -247,16 +282,52 @@ def prepare2d(grid, points, *, check_support=True):
     return Stencil2D((ids[0], ids[1]), (w[0], w[1]))
 
 
+def _pair_tables(stencil, like, values):
+    """The two components' (ids, weights) when the one-launch 2D transfers take
+    them: 16 taps per point, contiguous tables of matching types; else None."""
+    if len(stencil.indices) != 2 or len(stencil.weights) != 2 or like.dtype not in (torch.float32, torch.float64):
+        return None
+    shape = stencil.indices[0].shape
+    if len(shape) != 2 or shape[1] != 16:
+        return None
+    for ids, w in zip(stencil.indices, stencil.weights):
+        if not (ids.shape == shape and w.shape == shape and ids.dtype == torch.int64 and w.dtype == like.dtype
+                and ids.is_contiguous() and w.is_contiguous() and ids.device == like.device and w.device == like.device
+                and not w.requires_grad):
+            return None
+    if any(t.requires_grad or t.device != like.device or t.dtype != like.dtype for t in values):
+        return None
+    return (*stencil.indices, *stencil.weights)
+
+
 def spread2d(grid, force, stencil):
     """``TriangleTransfer._spread`` CUDA branch (``mac2d/transfer.py:108-112``):
     point forces (P,2) -> (u, v) face fields divided by the cell area."""
-    return tuple(indexed_spread(force[:, c:c + 1], stencil.indices[c], stencil.weights[c],
-                                grid.face_shape(c)[0] * grid.face_shape(c)[1], grid.volume)
+    sizes = [grid.face_shape(c)[0] * grid.face_shape(c)[1] for c in range(2)]
+    if torch.is_tensor(force) and force.is_cuda and force.dim() == 2 and force.shape[1] >= 2:
+        tables = _pair_tables(stencil, force, (force,))
+        if (tables is not None and tables[0].shape[0] == force.shape[0] and min(sizes) > 0
+                and 0 < grid.volume < float('inf')):
+            force = force.contiguous()
+            u, v = (torch.empty(grid.face_shape(c), device=force.device, dtype=force.dtype) for c in range(2))
+            call('afsi_b200_indexed_spread2', ptr(force), force.shape[1], *(ptr(t) for t in tables), force.shape[0],
+                 *sizes, float(grid.volume), ptr(u), ptr(v), ptr(_lib.status_word(force.device)),
+                 dtype_code(force.dtype), stream(force.device))
+            return u, v
+    return tuple(indexed_spread(force[:, c:c + 1], stencil.indices[c], stencil.weights[c], sizes[c], grid.volume)
                  .reshape(grid.face_shape(c)) for c in range(2))
 
 
 def gather2d(velocity, stencil):
     """``TriangleTransfer._gather`` CUDA branch (``mac2d/transfer.py:122-124``)."""
+    if len(velocity) == 2 and all(torch.is_tensor(u) and u.is_cuda and u.numel() > 0 for u in velocity):
+        tables = _pair_tables(stencil, velocity[0], velocity)
+        if tables is not None:
+            u, v = (t.contiguous() for t in velocity)
+            out = torch.empty((tables[0].shape[0], 2), device=u.device, dtype=u.dtype)
+            call('afsi_b200_indexed_gather2', ptr(u), ptr(v), u.numel(), v.numel(), *(ptr(t) for t in tables),
+                 out.shape[0], ptr(out), ptr(_lib.status_word(u.device)), dtype_code(u.dtype), stream(u.device))
+            return out
     return torch.cat([indexed_gather(u.reshape(-1, 1), ids, w)
                       for u, ids, w in zip(velocity, stencil.indices, stencil.weights)], -1)
 

@@ -267,8 +267,9 @@ class P1CSRTransfer:
         table, values in a fixed order.  None where the hash form is to be used:
         tables of another layout or type, more groups than one launch takes, a
         node id or support out of range (the hash form raises it), a row whose
-        box exceeds shared memory, or rows so much wider than their cells'
-        boxes that the padded rows would outgrow half the cells' entries."""
+        box exceeds shared memory, or (above 4 M entries) rows so much wider than
+        their cells' boxes that the padded rows would outgrow half the cells'
+        entries."""
         groups, base, phi = stencil.rule.groups, stencil.base, stencil.phi
         like, dev, lib = groups[0].weights, stencil.base.device, _lib.load()
         elements, nodes, shape = sum(g.cells.shape[0] for g in groups), self.node_count, self.grid.shape
@@ -300,7 +301,7 @@ class P1CSRTransfer:
         counts = info.tolist()
         sites, padded = counts[_lib.ROWS_SITES:_lib.ROWS_SITES + 3], counts[_lib.ROWS_PADDED:_lib.ROWS_PADDED + 3]
         cap = counts[_lib.ROWS_BOX]
-        if counts[_lib.ROWS_FLAGS] or not 0 < cap <= lib.afsi_b200_p1_rows_cap(code) or sum(padded) > 2 * sum(sites):
+        if counts[_lib.ROWS_FLAGS] or not 0 < cap <= lib.afsi_b200_p1_rows_cap(code) or sum(padded) > max(1 << 22, 2 * sum(sites)):
             return None
         pcol, pval = new(sum(padded), torch.int32), new(sum(padded), like.dtype)
         row_counts = volume  # the volumes are used up

@@ -300,6 +300,25 @@ int32_t afsi_b200_compact_gather(const void* field, const int64_t* base, const v
 int32_t afsi_b200_compact_spread(const void* field, const int64_t* base, const void* phi,
     int64_t points, int64_t nx, int64_t ny, int64_t nz, double volume, void* out,
     int32_t* status, int32_t dtype, afsi_stream_t stream);
+/* The three components of a staggered grid of (nx, ny, nz) cells in one
+ * launch: base (3, points, 3) and phi (3, points, 3, 4), point values
+ * (points, 3).  spread3 clears the face arrays first. */
+int32_t afsi_b200_compact_gather3(const void* u0, const void* u1, const void* u2, const int64_t* base,
+    const void* phi, int64_t points, int64_t nx, int64_t ny, int64_t nz, void* out, int32_t* status,
+    int32_t dtype, afsi_stream_t stream);
+int32_t afsi_b200_compact_spread3(const void* force, const int64_t* base, const void* phi, int64_t points,
+    int64_t nx, int64_t ny, int64_t nz, double volume, void* u0, void* u1, void* u2, int32_t* status,
+    int32_t dtype, afsi_stream_t stream);
+/* Both components of a 2D channel transfer in one launch, 16 taps per point:
+ * u (nu values) and v (nv), point values (points, 2) out of the gather, and
+ * `stride` >= 2 values per point into the spread, which clears u and v first. */
+int32_t afsi_b200_indexed_gather2(const void* u, const void* v, int64_t nu, int64_t nv, const int64_t* ids0,
+    const int64_t* ids1, const void* w0, const void* w1, int64_t points, void* out, int32_t* status,
+    int32_t dtype, afsi_stream_t stream);
+int32_t afsi_b200_indexed_spread2(const void* force, int64_t stride, const int64_t* ids0, const int64_t* ids1,
+    const void* w0, const void* w1, int64_t points, int64_t nu, int64_t nv, double volume, void* u, void* v,
+    int32_t* status, int32_t dtype, afsi_stream_t stream);
+
 
 /* P2 fused spread of one quadrature group (p2_spread_): for element e and
  * point q, F = (sum_a N[q,a]*value[cells[e,a]])*W[e,q], spread with the shared
