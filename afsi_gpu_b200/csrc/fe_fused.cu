@@ -36,6 +36,7 @@
 // support origin changes.  A point whose support leaves the grid sets
 // AFSI_FLAG_SUPPORT and is skipped; an element with a node id outside
 // [0, nodes) sets AFSI_FLAG_INDEX and is skipped.
+#include <algorithm>
 #include <climits>
 #include <cmath>
 #include <cub/device/device_radix_sort.cuh>
@@ -804,6 +805,384 @@ __global__ void __launch_bounds__(kGWarps * 32, 4) fused_gather_kernel(
     }
 }
 
+// ------------------------------------------------- several elements per warp
+//
+// Rules of few points (P1 orders 2 and 3 have 8 and 15 points, P2 order 3 has 15)
+// leave most lanes of a warp-per-element kernel idle while the rows are formed,
+// and flush a box per element although the boxes of neighbouring elements
+// nearly coincide.  The warp therefore takes G consecutive elements (element
+// lists come in mesh order): their points fill the lanes, and one box, the
+// union of theirs, is zeroed, accumulated and flushed once.  Where the union
+// does not fit (elements that are not neighbours) each element's box is
+// accumulated and flushed by itself from the same rows.
+//
+// Between components only two of the three rows of a point change (component c
+// reads axis a on lattice a != c: from 0 to 1 axes 0 and 1, from 1 to 2 axes 1
+// and 2), so the third is kept: 7 rows per point instead of 9, the same values.
+
+// Bound by instruction issue (64 % and 67 % active at 16 and 24 warps per SM).
+// 128,000 P1 elements of 8 and 15 points on 128^3, FP32 beside FP64 positions,
+// one B200: spread 677 -> 233 us (345 us with one box copy and a point per
+// warp step instead of a point per half-warp), gather-assemble 442 -> 126 us.
+// Lists of fewer than two elements per warp at 8 warps per SM keep the
+// warp-per-element kernels: there the idle SMs cost more than the idle lanes.
+
+constexpr int kMWarps = 4;
+constexpr int kMPoints = 64;    // spread: points per warp
+constexpr int kMBoxCap = 432;   // spread: entries of the padded union box (16 mod 32: the two FP32 copies are half the banks apart)
+constexpr int kMGPoints = 32;   // gather: one point per lane
+
+// Node positions (and values) of elements e0 .. e0+ne-1, ne * NPC <= 32, lane
+// per node; returns the elements whose node ids are all in range (bit el) and
+// flags the others.
+template <class TP, class T, int NPC>
+__device__ __forceinline__ unsigned stage_elements(const TP* __restrict__ x, const int64_t* __restrict__ cells,
+                                                   const T* __restrict__ value, int64_t e0, int ne, int64_t nodes,
+                                                   TP* xs, T* coef, int64_t& node, int32_t* status) {
+    const int lane = threadIdx.x & 31;
+    const bool mine = lane < ne * NPC;
+    node = mine ? cells[e0 * NPC + lane] : 0;
+    const bool in = node >= 0 && node < nodes;
+    const unsigned bad = __ballot_sync(0xffffffffu, mine && !in);
+    __syncwarp();
+    if (mine && in) {
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            xs[lane * 3 + d] = x[node * 3 + d];
+            if (value) coef[lane * 3 + d] = value[node * 3 + d];
+        }
+    }
+    unsigned ok = (1u << ne) - 1u;
+    if (bad) {
+        if (lane == 0) flag(status, AFSI_FLAG_INDEX);
+        for (int el = 0; el < ne; ++el)
+            if ((bad >> (el * NPC)) & ((1u << NPC) - 1u)) ok &= ~(1u << el);
+    }
+    __syncwarp();
+    return ok;
+}
+
+// Row of axis a on lattice l: support origin and, in r, the four weights.
+template <class TP>
+__device__ __forceinline__ int axis_row(const Geo<TP>& geo, TP pos, int a, int l, TP r[4]) {
+    const TP scaled = lattice_scaled(geo, pos, a, l);
+    const int64_t lower = static_cast<int64_t>(floor(scaled - TP(1)));
+    peskin_radical(scaled - TP(lower) - TP(1), r);
+    return int(lower);
+}
+
+template <class T>
+__device__ __forceinline__ void store_row(T* dst, const T w[4]) {  // dst 16-byte aligned
+    if constexpr (sizeof(T) == 8) {
+        reinterpret_cast<double2*>(dst)[0] = make_double2(w[0], w[1]);
+        reinterpret_cast<double2*>(dst)[1] = make_double2(w[2], w[3]);
+    } else {
+        *reinterpret_cast<float4*>(dst) = make_float4(w[0], w[1], w[2], w[3]);
+    }
+}
+
+template <class T>
+__device__ __forceinline__ void load_row(const T* src, T w[4]) {  // src 16-byte aligned
+    if constexpr (sizeof(T) == 8) {
+        const double2 a = reinterpret_cast<const double2*>(src)[0], b = reinterpret_cast<const double2*>(src)[1];
+        w[0] = a.x;
+        w[1] = a.y;
+        w[2] = b.x;
+        w[3] = b.y;
+    } else {
+        const float4 v = *reinterpret_cast<const float4*>(src);
+        w[0] = v.x;
+        w[1] = v.y;
+        w[2] = v.z;
+        w[3] = v.w;
+    }
+}
+
+// FP64 sums runs on the tensor cores into one box; FP32 adds point by point
+// into two copies (spread_points).
+template <class T> struct MCopies { static constexpr int value = sizeof(T) == 8 ? 1 : 2; };
+
+template <class TP, class T, int NPC>
+struct __align__(16) MStage {
+    T w[(kMPoints + 1) * 12];  // rows of the component: x at q*12, y at q*12+4, z at q*12+8; the last stays zero
+    T box[MCopies<T>::value * kMBoxCap];
+    T f[3][kMPoints + 1];      // force factors per component; the last stays zero
+    T coef[96];
+    TP xs[96];
+    int key[kMPoints];
+    int perm[4 * kMPoints];
+    int rs[kMPoints + 1], rk[kMPoints];
+};
+
+// Adds points 0..n-1 to the box copies, two at a time: half-warp h takes points
+// h, h + 2, ... into copy h, its lane (i, j) the link column (i, j) with the four
+// z links.  at[q]: offset of the support origin in the box, or -1.
+template <class T>
+__device__ __forceinline__ void spread_points(T* box, int copy, const int* at, const T* f, const T* w, int n, int sx,
+                                              int sy) {
+    const int lane = threadIdx.x & 31, half = lane >> 4, li = (lane >> 2) & 3, lj = lane & 3;
+    T* const mine = box + half * copy + li * sx + lj * sy;
+    for (int q = half; q < n + half; q += 2) {  // the same trip count in both halves
+        const int k = q < n ? at[q] : -1;
+        if (k >= 0) {
+            const T* row = w + q * 12;
+            const T a = (row[li] * row[4 + lj]) * f[q];
+            T z[4];
+            load_row(row + 8, z);
+            T* dst = mine + k;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) dst[i] = fma(a, z[i], dst[i]);
+        }
+        __syncwarp();
+    }
+}
+
+template <class TP, class T, int NPC>
+__global__ void __launch_bounds__(kMWarps * 32, 4) fused_spread_multi_kernel(
+    const TP* __restrict__ x, const int64_t* __restrict__ cells, const TP* __restrict__ Npos, const T* __restrict__ N,
+    const T* __restrict__ W, const T* __restrict__ value, Geo<TP> geo, T* __restrict__ u0, T* __restrict__ u1,
+    T* __restrict__ u2, FusedDims g, int G, T volume, T inv_volume, int32_t* status) {
+    extern __shared__ __align__(16) unsigned char fused_smem[];
+    MStage<TP, T, NPC>& s = reinterpret_cast<MStage<TP, T, NPC>*>(fused_smem)[threadIdx.x >> 5];
+    constexpr int C = kMPoints, J = C / 32;
+    const int lane = threadIdx.x & 31;
+    const int nq = int(g.nq);
+    const int64_t items = (g.elements + G - 1) / G, warps = int64_t(gridDim.x) * kMWarps;
+    if (lane < 12) s.w[C * 12 + lane] = T(0);
+    if (lane < 3) s.f[lane][C] = T(0);
+    for (int64_t it = int64_t(blockIdx.x) * kMWarps + (threadIdx.x >> 5); it < items; it += warps) {
+        const int64_t e0 = it * G;
+        const int ne = int(g.elements - e0 < G ? g.elements - e0 : G), n = ne * nq;
+        int64_t node;
+        const unsigned ok = stage_elements<TP, T, NPC>(x, cells, value, e0, ne, g.nodes, s.xs, s.coef, node, status);
+        TP pos[J][3];
+        int el[J], b[J][3];
+        bool live[J];
+#pragma unroll
+        for (int j = 0; j < J; ++j) {
+            const int p = lane + 32 * j;
+            live[j] = false;
+            el[j] = 0;
+            if (p < n) {
+                el[j] = p / nq;
+                const int q = p - el[j] * nq;
+                if ((ok >> el[j]) & 1u) {
+                    live[j] = point_position<TP, NPC>(Npos, s.xs + el[j] * NPC * 3, q, geo, pos[j]);
+                    if (!live[j]) flag(status, AFSI_FLAG_SUPPORT);
+                    T F[3] = {T(0), T(0), T(0)};
+#pragma unroll
+                    for (int a = 0; a < NPC; ++a) {
+                        const T nv = N[q * NPC + a];
+#pragma unroll
+                        for (int c = 0; c < 3; ++c) F[c] += nv * s.coef[(el[j] * NPC + a) * 3 + c];
+                    }
+                    const T wq = W[e0 * nq + p];
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) {
+                        const T fw = F[c] * wq;
+                        s.f[c][p] = inv_volume != T(0) ? fw * inv_volume : fw / volume;
+                    }
+                }
+            }
+        }
+#pragma unroll 1
+        for (int c = 0; c < 3; ++c) {
+            T* field = c == 0 ? u0 : c == 1 ? u1 : u2;
+            int mn[3], mx[3];
+            bounds_init(mn, mx);
+#pragma unroll
+            for (int j = 0; j < J; ++j) {
+                if (!live[j]) continue;
+                T* row = s.w + (lane + 32 * j) * 12;
+#pragma unroll
+                for (int a = 0; a < 3; ++a) {
+                    if (c > 0 && a == (c == 1 ? 2 : 0)) continue;  // the row of the previous component
+                    TP r[4];
+                    b[j][a] = axis_row(geo, pos[j][a], a, a != c, r);
+                    const T w[4] = {T(r[0]), T(r[1]), T(r[2]), T(r[3])};
+                    store_row(row + a * 4, w);
+                }
+                bounds_add(mn, mx, b[j]);
+            }
+            FBox bx;
+            if (!bounds_finish(mn, mx, bx)) continue;  // no valid point
+            int sx = 0, sy = 0;
+            bool fits = fbox_layout(bx, g, c, sx, sy, kMBoxCap);
+            const int parts = fits ? 1 : ne;
+            for (int part = 0; part < parts; ++part) {
+                if (parts > 1) {  // element `part` alone
+                    bounds_init(mn, mx);
+#pragma unroll
+                    for (int j = 0; j < J; ++j)
+                        if (live[j] && el[j] == part) bounds_add(mn, mx, b[j]);
+                    if (!bounds_finish(mn, mx, bx)) continue;
+                    fits = fbox_layout(bx, g, c, sx, sy, kMBoxCap);
+                }
+                if (fits) {
+                    constexpr bool mma = sizeof(T) == 8;
+                    const int size = bx.ext[0] * sx;
+                    for (int t = lane; t < size; t += 32) {
+                        s.box[t] = T(0);
+                        if (!mma) s.box[kMBoxCap + t] = T(0);
+                    }
+#pragma unroll
+                    for (int j = 0; j < J; ++j) {
+                        const int p = lane + 32 * j, d0 = b[j][0] - bx.lo[0], d1 = b[j][1] - bx.lo[1],
+                                  d2 = b[j][2] - bx.lo[2];
+                        if (p < n)
+                            s.key[p] = live[j] && (parts == 1 || el[j] == part)
+                                           ? (mma ? run_key(d0, d1, d2) : d0 * sx + d1 * sy + d2)
+                                           : -1;
+                    }
+                    __syncwarp();
+                    if constexpr (mma)
+                        spread_runs_mma<C>(s.box, s.key, s.f[c], s.w, s.w + 4, s.w + 8, n, sx, sy, s.perm, s.rs, s.rk);
+                    else
+                        spread_points(s.box, kMBoxCap, s.key, s.f[c], s.w, n, sx, sy);
+                    __syncwarp();
+                    fbox_walk(lane, bx.ext[0], bx.ext[1], bx.ext[2], [&](int xx, int yy, int zz) {
+                        const int o = xx * sx + yy * sy + zz;
+                        const T v = mma ? s.box[o] : s.box[o] + s.box[kMBoxCap + o];
+                        if (v != T(0))
+                            atomicAdd(field + ffield_index(g, c, bx.lo[0] + xx, bx.lo[1] + yy, bx.lo[2] + zz), v);
+                    });
+                    __syncwarp();
+                } else {  // the element's own box leaves the array or the cap: its points one by one
+#pragma unroll
+                    for (int j = 0; j < J; ++j) {
+                        if (!live[j] || (parts > 1 && el[j] != part)) continue;
+                        const int p = lane + 32 * j;
+                        if (!fpoint_inside(g, c, b[j][0], b[j][1], b[j][2])) {
+                            flag(status, AFSI_FLAG_INDEX);
+                            continue;
+                        }
+                        const T* w = s.w + p * 12;
+                        T* dst = field + ffield_index(g, c, b[j][0], b[j][1], b[j][2]);
+                        const int64_t fz = g.nz + (c == 2), fy = (g.ny + (c == 1)) * fz;
+                        for (int i = 0; i < 4; ++i)
+                            for (int jj = 0; jj < 4; ++jj) {
+                                const T a = (w[i] * w[4 + jj]) * s.f[c][p];
+                                for (int k = 0; k < 4; ++k) atomicAdd(dst + i * fy + jj * fz + k, a * w[8 + k]);
+                            }
+                    }
+                    __syncwarp();
+                }
+            }
+        }
+        __syncwarp();
+    }
+}
+
+template <class TP, class T, int NPC>
+struct __align__(16) MGStage {
+    T patch[kGPatch];
+    T u[3][kMGPoints];
+    T w[kMGPoints];
+    TP xs[96];
+};
+
+template <class TP, class T, int NPC, bool Local>
+__global__ void __launch_bounds__(kMWarps * 32, 6) fused_gather_multi_kernel(
+    const T* __restrict__ u0, const T* __restrict__ u1, const T* __restrict__ u2, const TP* __restrict__ x,
+    const int64_t* __restrict__ cells, const TP* __restrict__ Npos, const T* __restrict__ N, const T* __restrict__ W,
+    Geo<TP> geo, T* __restrict__ out, FusedDims g, int G, int32_t* status) {
+    extern __shared__ __align__(16) unsigned char fused_smem[];
+    MGStage<TP, T, NPC>& s = reinterpret_cast<MGStage<TP, T, NPC>*>(fused_smem)[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31;
+    const int nq = int(g.nq);
+    const int64_t items = (g.elements + G - 1) / G, warps = int64_t(gridDim.x) * kMWarps;
+    for (int64_t it = int64_t(blockIdx.x) * kMWarps + (threadIdx.x >> 5); it < items; it += warps) {
+        const int64_t e0 = it * G;
+        const int ne = int(g.elements - e0 < G ? g.elements - e0 : G), n = ne * nq;
+        int64_t node;
+        const unsigned ok = stage_elements<TP, T, NPC>(x, cells, static_cast<const T*>(nullptr), e0, ne, g.nodes, s.xs,
+                                                       static_cast<T*>(nullptr), node, status);
+        TP pos[3];
+        bool live = false;
+        if (lane < n) {
+            const int el = lane / nq, q = lane - el * nq;
+            if ((ok >> el) & 1u) {
+                live = point_position<TP, NPC>(Npos, s.xs + el * NPC * 3, q, geo, pos);
+                if (!live) flag(status, AFSI_FLAG_SUPPORT);
+            }
+            s.w[lane] = W[e0 * nq + lane];
+        }
+        T wr[3][4];
+        int b[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const T* field = c == 0 ? u0 : c == 1 ? u1 : u2;
+            int mn[3], mx[3];
+            bounds_init(mn, mx);
+            if (live) {
+#pragma unroll
+                for (int a = 0; a < 3; ++a) {
+                    if (c > 0 && a == (c == 1 ? 2 : 0)) continue;  // the row of the previous component
+                    TP r[4];
+                    b[a] = axis_row(geo, pos[a], a, a != c, r);
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) wr[a][k] = T(r[k]);
+                }
+                bounds_add(mn, mx, b);
+            }
+            FBox bx;
+            bool fits = bounds_finish(mn, mx, bx);
+            const int64_t fe[3] = {g.nx + (c == 0), g.ny + (c == 1), g.nz + (c == 2)};
+#pragma unroll
+            for (int a = 0; a < 3; ++a)
+                fits = fits && bx.lo[a] >= 0 && int64_t(bx.lo[a]) + bx.ext[a] <= fe[a] && bx.ext[a] <= kGExt;
+            __syncwarp();  // the previous component's patch reads are done
+            if (fits)
+                fbox_walk(lane, bx.ext[0], bx.ext[1], bx.ext[2], [&](int xx, int yy, int zz) {
+                    s.patch[xx * kGSX + yy * kGSY + zz] =
+                        field[ffield_index(g, c, bx.lo[0] + xx, bx.lo[1] + yy, bx.lo[2] + zz)];
+                });
+            __syncwarp();
+            if (lane < n) {
+                T U = T(0);
+                if (live) {
+                    if (fits) {
+                        U = support_dot(s.patch + (b[0] - bx.lo[0]) * kGSX + (b[1] - bx.lo[1]) * kGSY + (b[2] - bx.lo[2]),
+                                        kGSX, kGSY, wr[0], wr[1], wr[2]);
+                    } else if (fpoint_inside(g, c, b[0], b[1], b[2])) {
+                        const int64_t sz = g.nz + (c == 2), sy = (g.ny + (c == 1)) * sz;
+                        U = support_dot(field + ffield_index(g, c, b[0], b[1], b[2]), sy, sz, wr[0], wr[1], wr[2]);
+                    } else {
+                        flag(status, AFSI_FLAG_INDEX);
+                    }
+                }
+                s.u[c][lane] = U;
+            }
+        }
+        __syncwarp();
+        // nodal sums, lanes over (element, node, component)
+        for (int o0 = 0; o0 < ne * NPC * 3; o0 += 32) {
+            const int o = o0 + lane, slot = o / 3, cc = o - 3 * slot;
+            const int64_t nd = __shfl_sync(0xffffffffu, node, slot & 31);
+            if (o < ne * NPC * 3) {
+                const int el = slot / NPC, a = slot - el * NPC;
+                if ((ok >> el) & 1u) {
+                    T acc = T(0);
+                    for (int q = 0; q < nq; ++q) acc = fma(N[q * NPC + a] * s.w[el * nq + q], s.u[cc][el * nq + q], acc);
+                    if (Local)
+                        out[((e0 + el) * NPC + a) * 3 + cc] = acc;
+                    else
+                        atomicAdd(out + nd * 3 + cc, acc);
+                }
+            }
+        }
+        __syncwarp();
+    }
+}
+
+// Elements per warp: as many as fill `points` lanes' worth of points and the
+// lanes with nodes, while at least 8 warps per SM of a B200 are left; 1 takes
+// the warp-per-element kernels.
+inline int elements_per_warp(int64_t elements, int64_t nq, int npc, int points) {
+    const int64_t most = std::min<int64_t>(points / nq, 32 / npc);
+    return int(std::max<int64_t>(1, std::min<int64_t>(most, elements / (148 * 8))));
+}
+
 template <class TP>
 Geo<TP> make_geo(const double* origin, const double* spacing, const double* limits) {
     Geo<TP> geo;
@@ -880,6 +1259,26 @@ extern "C" int32_t afsi_b200_fe_fused_spread(int32_t nodes_per_cell, const void*
     const FusedDims g{nx, ny, nz, nodes, elements, nq};
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     AFSI_FUSED_DISPATCH(nodes_per_cell, pos_dtype, dtype, {
+        const int G = elements_per_warp(elements, nq, NPC, kMPoints);
+        if (G > 1) {
+            const size_t multi = sizeof(MStage<TP, T, NPC>) * kMWarps;
+            static bool multi_configured = false;  // once per instantiation, before any graph capture of it
+            if (!multi_configured) {
+                cudaFuncSetAttribute(fused_spread_multi_kernel<TP, T, NPC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     int(multi));
+                multi_configured = true;
+            }
+            const T vol = T(volume);
+            int ex = 0;
+            const bool pow2 = std::frexp(double(vol), &ex) == 0.5 && std::isnormal(T(1) / vol);
+            fused_spread_multi_kernel<TP, T, NPC>
+                <<<fused_blocks((elements + G - 1) / G, kMWarps), kMWarps * 32, multi, s>>>(
+                    static_cast<const TP*>(x), cells, static_cast<const TP*>(N_pos), static_cast<const T*>(N),
+                    static_cast<const T*>(W), static_cast<const T*>(value), make_geo<TP>(origin, spacing, limits),
+                    static_cast<T*>(u0), static_cast<T*>(u1), static_cast<T*>(u2), g, G, vol, pow2 ? T(1) / vol : T(0),
+                    status);
+            return launched("fused_spread_multi");
+        }
         const size_t smem = sizeof(FStage<TP, T, NPC>) * kFWarps;
         static bool configured = false;  // once per instantiation, before any graph capture of it
         if (!configured) {
@@ -1003,6 +1402,22 @@ static int32_t fused_gather(int32_t nodes_per_cell, const void* x, int64_t nodes
     const FusedDims g{nx, ny, nz, nodes, elements, nq};
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     AFSI_FUSED_DISPATCH(nodes_per_cell, pos_dtype, dtype, {
+        const int G = elements_per_warp(elements, nq, NPC, kMGPoints);
+        if (G > 1) {
+            const size_t multi = sizeof(MGStage<TP, T, NPC>) * kMWarps;
+            static bool multi_configured = false;  // once per instantiation, before any graph capture of it
+            if (!multi_configured) {
+                cudaFuncSetAttribute(fused_gather_multi_kernel<TP, T, NPC, Local>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, int(multi));
+                multi_configured = true;
+            }
+            fused_gather_multi_kernel<TP, T, NPC, Local>
+                <<<fused_blocks((elements + G - 1) / G, kMWarps), kMWarps * 32, multi, s>>>(
+                    static_cast<const T*>(u0), static_cast<const T*>(u1), static_cast<const T*>(u2),
+                    static_cast<const TP*>(x), cells, static_cast<const TP*>(N_pos), static_cast<const T*>(N),
+                    static_cast<const T*>(W), make_geo<TP>(origin, spacing, limits), static_cast<T*>(out), g, G, status);
+            return launched(Local ? "fused_gather_local_multi" : "fused_gather_multi");
+        }
         const size_t smem = sizeof(FGStage<TP, T, NPC>) * kGWarps;
         static bool configured = false;  // once per instantiation, before any graph capture of it
         if (!configured) {
