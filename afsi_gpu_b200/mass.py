@@ -164,8 +164,10 @@ class MassSolver:
             if self._graph is not None:
                 _lib.call('afsi_b200_pcg_graph_launch', self._graph, s)
                 state = self._read()
-                # the WHILE body ran once per iteration (once, as no-ops, when begin stopped the solve)
-                _lib.count_replay(self.graph_body_launches * max(int(state[_ITERATIONS]), 1))
+                # the WHILE body holds several iterations of three launches (one body of no-ops when begin
+                # stopped the solve)
+                per_body = self.graph_body_launches // 3
+                _lib.count_replay(self.graph_body_launches * -(-max(int(state[_ITERATIONS]), 1) // per_body))
             else:
                 state = self._read()
                 iteration = 0
