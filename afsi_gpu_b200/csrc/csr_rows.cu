@@ -13,22 +13,25 @@
 //              shared by the three components;
 //   fill       one warp per (component, node): the union box in shared memory,
 //              the points of the node's cells in order (32 points staged at a
-//              time, whichever cells they belong to), each added link by link;
+//              time, whichever cells they belong to): FP64 sums the points of
+//              one support origin on the tensor cores (spread_runs_mma) and
+//              adds each sum, FP32 adds point by point;
 //              the touched entries leave the box in ascending face order, which
 //              is the CSR column order: B needs no sort.  An entry exists when
-//              some point's contribution is nonzero (untouched entries hold -0,
-//              which no sum of nonzero terms gives);
+//              some contribution is nonzero (untouched entries hold -0, which no
+//              sum of nonzero terms gives);
 //   finish     the padded rows packed to CSR, and the transpose by a stable
 //              radix sort on the face index alone (32-bit keys and positions).
 //
 // No atomics on values: the operators are the same bit for bit on every run.
-// What bounds it: the fill is bound by instruction issue and shared-memory
-// read-modify-writes (64 links per point and component, each cell visited by
-// its four nodes); the finish by the HBM passes of the sort.  128,000
-// tetrahedra (1.2 M points) on 128^3, FP64, one B200: fill 1.04 ms, sorts
-// 0.39 ms, pack and transpose 0.29 ms for the three components, where the hash
-// contraction took 4.98 ms and the table's sorts 2.57 ms; tables, assembly,
-// spread and interpolate together 9.64 -> 2.67 ms.
+// What bounds it: the fill is bound by shared memory (64 links per point and
+// component, each cell visited by its four nodes; adding every point by itself
+// kept the shared-memory pipe 80 % busy), the finish by the HBM passes of the
+// sort.  128,000 tetrahedra (1.2 M points) on 128^3, FP64, one B200: fill
+// 0.80 ms (1.04 ms point by point), sorts 0.39 ms, pack and transpose 0.29 ms
+// for the three components, where the hash contraction took 4.98 ms and the
+// table's sorts 2.57 ms; tables, assembly, spread and interpolate together
+// 9.64 -> 2.39 ms.
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
 #include <algorithm>
@@ -210,9 +213,10 @@ struct RowGroups {
 // Staged points and the cells they come from, per warp; the box follows.
 template <class T>
 struct __align__(16) RowsStage {
-    T w[32 * 12];      // weight rows: x, y, z, four each
-    T f[32];           // W N[q,a]
-    int at[32];        // offset of the support origin in the box
+    T w[33 * 12];      // weight rows: x, y, z, four each; the last stays zero
+    T f[33];           // W N[q,a]; the last stays zero
+    int at[32];        // FP64: run key of the support origin in the box, FP32: its offset
+    int perm[128], rs[33], rk[32];  // FP64: runs of one origin
     int pre[33];       // first point of each of the 32 current cells
     int grp[32];
     int64_t e4a[32];   // (element within its group) * 4 + a
@@ -228,8 +232,8 @@ template <> struct Neg0<float> {
 
 // Rows of B: one warp per (component, node), 4 warps per block.  `cap` is the
 // largest padded box of any row (entries of dynamic shared memory per warp).
-// Lane (half, i, j) owns the link column (i, j) and z links 2 half, 2 half + 1
-// of each point; the padded strides keep a half-warp's 16 columns in distinct
+// FP32: lane (half, i, j) owns the link column (i, j) and z links 2 half,
+// 2 half + 1 of each point; the padded strides keep a half-warp's 16 columns in distinct
 // banks, and the links of one point are distinct entries, so the adds are
 // plain read-modify-writes in point order.
 template <class T>
@@ -246,6 +250,9 @@ __global__ void __launch_bounds__(kRowsWarps * 32) rows_fill_kernel(
     const int lane = threadIdx.x & 31, half = lane >> 4, li = (lane >> 2) & 3, lj = lane & 3;
     const int c = blockIdx.y;
     const int64_t warps = int64_t(gridDim.x) * kRowsWarps;
+    constexpr bool mma = sizeof(T) == 8;
+    if (lane < 12) s.w[32 * 12 + lane] = T(0);
+    if (lane == 0) s.f[32] = T(0);
     using P = typename std::conditional<sizeof(T) == 8, double2, float2>::type;
     for (int64_t n = int64_t(blockIdx.x) * kRowsWarps + (threadIdx.x >> 5); n < nodes; n += warps) {
         const int4 nb = node_box[int64_t(c) * nodes + n];
@@ -300,7 +307,7 @@ __global__ void __launch_bounds__(kRowsWarps * 32) rows_fill_kernel(
 #pragma unroll
                     for (int a = 0; a < 3; ++a) {
                         const int64_t r = (int64_t(a != c) * total + r0) * 3 + a;
-                        at += (int(base[r]) - lo[a]) * st[a];
+                        at += mma ? (int(base[r]) - lo[a]) << (10 * a) : (int(base[r]) - lo[a]) * st[a];
                         const P w0 = reinterpret_cast<const P*>(phi + r * 4)[0], w1 = reinterpret_cast<const P*>(phi + r * 4)[1];
                         row[a * 4] = w0.x;
                         row[a * 4 + 1] = w0.y;
@@ -322,7 +329,9 @@ __global__ void __launch_bounds__(kRowsWarps * 32) rows_fill_kernel(
                     s.at[lane] = at;
                 }
                 __syncwarp();
-                for (int j = 0; j < m; ++j) {
+                if constexpr (mma) {
+                    spread_runs_mma<32, true>(acc, s.at, s.f, s.w, s.w + 4, s.w + 8, m, sx, sy, s.perm, s.rs, s.rk);
+                } else for (int j = 0; j < m; ++j) {
                     const T* w = s.w + j * 12;
                     const T a = (w[li] * w[4 + lj]) * s.f[j];
                     const P z = *reinterpret_cast<const P*>(w + 8 + 2 * half);

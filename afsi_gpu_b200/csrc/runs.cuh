@@ -132,8 +132,9 @@ __device__ __forceinline__ void mma884(double d[2], double a, double b) {
 // points at a time by two m8n8k4 steps (j = 0-1 and j = 2-3; rows 4-7 of A
 // read the zero row).  Lanes 0-15 then add their two pairs of z links to the
 // box.  Row `zero` (index C) of wx/wy/wz and f must be all zero; perm, rs and
-// rk are group_runs' scratch.
-template <int C>
+// rk are group_runs' scratch.  Touch: entries whose run sum is zero are left as
+// they are (a box that marks its untouched entries).
+template <int C, bool Touch = false>
 __device__ __forceinline__ void spread_runs_mma(double* box, const int* key, const double* f, const double* wx,
                                                 const double* wy, const double* wz, int n, int sx, int sy,
                                                 int* perm, int* rs, int* rk) {
@@ -157,11 +158,11 @@ __device__ __forceinline__ void spread_runs_mma(double* box, const int* key, con
         if (row < 4) {
             const int j0 = slot >> 1, k0 = 2 * (slot & 1);
             double* dst = box + ((K & 1023) + row) * sx + (((K >> 10) & 1023) + j0) * sy + (K >> 20) + k0;
-            dst[0] += d0[0];
-            dst[1] += d0[1];
+            if (!Touch || d0[0] != 0.0) dst[0] += d0[0];
+            if (!Touch || d0[1] != 0.0) dst[1] += d0[1];
             dst += 2 * sy;
-            dst[0] += d1[0];
-            dst[1] += d1[1];
+            if (!Touch || d1[0] != 0.0) dst[0] += d1[0];
+            if (!Touch || d1[1] != 0.0) dst[1] += d1[1];
         }
         __syncwarp();
     }
