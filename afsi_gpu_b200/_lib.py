@@ -193,6 +193,9 @@ _SIGNATURES = {
                                           c_int32, c_void_p],
     'afsi_b200_stokes_precondition_result': [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, P_I64,
                                              P_F64, c_double, c_double, c_int32, c_void_p],
+    'afsi_b200_krylov_scratch_bytes': [c_int64],
+    'afsi_b200_krylov_step': [c_void_p, c_int64, c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int32,
+                              c_void_p],
     'afsi_b200_batch2d_prepare': [c_void_p, c_int64, c_void_p, c_int32, c_void_p, c_void_p, c_void_p, c_int32,
                                   c_void_p],
     'afsi_b200_batch2d_spread': [c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_int32, c_void_p, c_void_p,
@@ -230,7 +233,7 @@ _RESTYPES = {'afsi_b200_last_error': ctypes.c_char_p, 'afsi_b200_mg_scratch_byte
              'afsi_b200_p1_plan_scratch_bytes': ctypes.c_int64, 'afsi_b200_hash_csr_scratch_bytes': ctypes.c_int64,
              'afsi_b200_pcg_scratch_bytes': ctypes.c_int64, 'afsi_b200_mg_refine_scratch_bytes': ctypes.c_int64,
              'afsi_b200_stokes_partial_blocks': ctypes.c_int64, 'afsi_b200_cache_scratch_bytes': ctypes.c_int64,
-             'afsi_b200_p1_rows_cap': ctypes.c_int64, 'afsi_b200_p1_rows_scratch_bytes': ctypes.c_int64,
+             'afsi_b200_p1_rows_cap': ctypes.c_int64, 'afsi_b200_krylov_scratch_bytes': ctypes.c_int64, 'afsi_b200_p1_rows_scratch_bytes': ctypes.c_int64,
              'afsi_b200_det_plan_bytes': ctypes.c_int64, 'afsi_b200_fe_det_spread_bytes': ctypes.c_int64}
 
 

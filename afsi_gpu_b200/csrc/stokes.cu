@@ -8,7 +8,7 @@
 //   sweep       out_c = u + (r - u + alpha L_c u)/diag_c, 0 on the walls, with
 //               L_c the face Laplacian whose missing neighbours are odd ghosts
 //               (-u), summed x, y, z (mac/grid.py:96-105).
-// All three face lattices in one launch (a flat index over the three arrays).
+// All three face lattices in one launch (grid y: component and x chunk).
 //
 // Stokes reductions (mac/_triton_stokes.py:8-145): one partial per 256 cells,
 // in the layouts the reference's reductions consume (mac/stokes_workspace.py):
@@ -21,6 +21,8 @@
 //   pressure norm   [sum rhs^2, sum (rhs - A p)^2] with the Neumann operator.
 // The library is built with --fmad=false, so every expression rounds as the
 // reference's fusion-free kernels do; block sums are a fixed tree.
+#include <algorithm>
+#include <cmath>
 #include "common.cuh"
 
 namespace afsi {
@@ -50,72 +52,107 @@ struct ConstFaces {
     __device__ __forceinline__ const T* at(int c) const { return c == 0 ? f[0] : (c == 1 ? f[1] : f[2]); }
 };
 
-// Flat index over the three face arrays back to back -> (component, local index).
-__device__ __forceinline__ int split_faces(const Cells& g, int64_t t, int64_t* local) {
-    const int64_t n0 = (g.nx + 1) * g.ny * g.nz, n1 = g.nx * (g.ny + 1) * g.nz;
-    if (t < n0) {
-        *local = t;
-        return 0;
-    }
-    if (t < n0 + n1) {
-        *local = t - n0;
-        return 1;
-    }
-    *local = t - n0 - n1;
-    return 2;
+// Launch geometry of the face kernels: a thread owns one (y, z) column of one
+// component (flat index over the plane, one 32-bit division per thread) and
+// marches `planes` planes along x, so a sweep reads each value of u once per
+// column instead of three times and recomputes no coordinates.
+struct March {
+    int n[3];       // face extents of the block's component
+    int y, z, x0, x1;
+    int64_t i;      // index of (x0, y, z)
+    int c;
+    bool active;
+};
+
+__device__ __forceinline__ March march_of(const Cells& g, int chunks) {
+    March m;
+    m.c = int(blockIdx.y) / chunks;
+    const int chunk = int(blockIdx.y) - m.c * chunks;
+    m.n[0] = int(g.nx) + (m.c == 0);
+    m.n[1] = int(g.ny) + (m.c == 1);
+    m.n[2] = int(g.nz) + (m.c == 2);
+    const int planes = (m.n[0] + chunks - 1) / chunks;
+    const unsigned t = blockIdx.x * 256u + threadIdx.x;  // planes below 2^32 faces
+    m.y = int(t / unsigned(m.n[2]));
+    m.z = int(t - unsigned(m.y) * unsigned(m.n[2]));
+    m.x0 = chunk * planes;
+    m.x1 = min(m.x0 + planes, m.n[0]);
+    m.i = (int64_t(m.x0) * m.n[1] + m.y) * m.n[2] + m.z;
+    m.active = m.y < m.n[1] && m.x0 < m.x1;
+    return m;
 }
 
 template <class T>
 __global__ void __launch_bounds__(256) helmholtz_initialize_kernel(ConstFaces<T> b, const T* __restrict__ p,
                                                                    ConstFaces<T> diag, Faces<T> rhs, Faces<T> u,
-                                                                   const T* __restrict__ param, Cells g,
-                                                                   double hx, double hy, double hz, int64_t total) {
-    const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (t >= total) return;
-    int64_t i;
-    const int c = split_faces(g, t, &i);
-    int64_t n[3];
-    face_dims(g, c, n);
-    const int64_t x = i / (n[1] * n[2]), y = (i / n[2]) % n[1], z = i % n[2];
-    const int64_t coord = c == 0 ? x : (c == 1 ? y : z);
-    const bool interior = coord > 0 && coord < n[c] - 1;
-    T r = b.at(c)[i];
-    if (p && interior) {
-        // pressure cells on either side of the face
-        const int64_t right = (x * g.ny + y) * g.nz + z;
-        const int64_t stride = c == 0 ? g.ny * g.nz : (c == 1 ? g.nz : 1);
-        const T h = T(c == 0 ? hx : (c == 1 ? hy : hz));
-        r = r - param[1] * ((p[right] - p[right - stride]) / h);
+                                                                   const T* __restrict__ param, Cells g, double hx,
+                                                                   double hy, double hz, int chunks) {
+    pdl_enter();
+    const March m = march_of(g, chunks);
+    if (!m.active) return;
+    const T* B = b.at(m.c) + m.i;
+    const T* D = diag.at(m.c) + m.i;
+    T *R = rhs.at(m.c) + m.i, *U = u.at(m.c) + m.i;
+    const int64_t sx = int64_t(m.n[1]) * m.n[2];
+    const T h = T(m.c == 0 ? hx : (m.c == 1 ? hy : hz));
+    const int64_t stride = m.c == 0 ? g.ny * g.nz : (m.c == 1 ? g.nz : 1);  // pressure cells on either side of the face
+    for (int x = m.x0; x < m.x1; ++x) {
+        const int coord = m.c == 0 ? x : (m.c == 1 ? m.y : m.z);
+        const int last = m.c == 0 ? m.n[0] : (m.c == 1 ? m.n[1] : m.n[2]);
+        const bool interior = coord > 0 && coord < last - 1;
+        T r = B[0];
+        if (p && interior) {
+            const int64_t right = (int64_t(x) * g.ny + m.y) * g.nz + m.z;
+            r = r - param[1] * ((p[right] - p[right - stride]) / h);
+        }
+        if (!interior) r = T(0);
+        R[0] = r;
+        U[0] = r / D[0];
+        B += sx;
+        D += sx;
+        R += sx;
+        U += sx;
     }
-    if (!interior) r = T(0);
-    rhs.at(c)[i] = r;
-    u.at(c)[i] = r / diag.at(c)[i];
 }
 
+// One sweep.  ih2[a]: 1/h_a^2 where h_a^2 is a power of two (the product then
+// rounds as the quotient does), else 0.  Bound by the L2 (u, rhs, diag in, u
+// out, 26 MB at 64^3) and, at 64^3, by the launch: 12.8 us with a thread per
+// face and three 64-bit divisions for its coordinates, 9.7 us with the
+// marching columns and programmatic dependent launch.
 template <class T>
 __global__ void __launch_bounds__(256) helmholtz_sweep_kernel(ConstFaces<T> u, ConstFaces<T> rhs, ConstFaces<T> diag,
                                                               Faces<T> out, const T* __restrict__ param, Cells g,
-                                                              double hx2, double hy2, double hz2, int64_t total) {
-    const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (t >= total) return;
-    int64_t i;
-    const int c = split_faces(g, t, &i);
-    int64_t n[3];
-    face_dims(g, c, n);
-    const int64_t x = i / (n[1] * n[2]), y = (i / n[2]) % n[1], z = i % n[2];
-    const T* U = u.at(c);
-    const T v = U[i];
-    const int64_t sx = n[1] * n[2], sy = n[2];
-    const T xm = x > 0 ? U[i - sx] : -v, xp = x + 1 < n[0] ? U[i + sx] : -v;
-    const T ym = y > 0 ? U[i - sy] : -v, yp = y + 1 < n[1] ? U[i + sy] : -v;
-    const T zm = z > 0 ? U[i - 1] : -v, zp = z + 1 < n[2] ? U[i + 1] : -v;
-    T lap = (xm - T(2) * v + xp) / T(hx2);
-    lap = lap + (ym - T(2) * v + yp) / T(hy2);
-    lap = lap + (zm - T(2) * v + zp) / T(hz2);
-    T value = v + (rhs.at(c)[i] - v + param[0] * lap) / diag.at(c)[i];
-    const int64_t coord = c == 0 ? x : (c == 1 ? y : z);
-    if (!(coord > 0 && coord < n[c] - 1)) value = T(0);
-    out.at(c)[i] = value;
+                                                              T hx2, T hy2, T hz2, T ihx2, T ihy2, T ihz2, int chunks) {
+    pdl_enter();
+    const March m = march_of(g, chunks);
+    if (!m.active) return;
+    const T alpha = param[0];
+    const T *U = u.at(m.c) + m.i, *R = rhs.at(m.c) + m.i, *D = diag.at(m.c) + m.i;
+    T* O = out.at(m.c) + m.i;
+    const int sy = m.n[2];
+    const int64_t sx = int64_t(m.n[1]) * m.n[2];
+    const bool ym_in = m.y > 0, yp_in = m.y + 1 < m.n[1], zm_in = m.z > 0, zp_in = m.z + 1 < m.n[2];
+    const bool wall = (m.c == 1 && !(ym_in && yp_in)) || (m.c == 2 && !(zm_in && zp_in));
+    T v = U[0], before = m.x0 > 0 ? U[-sx] : T(0);
+    for (int x = m.x0; x < m.x1; ++x) {
+        const T xp = x + 1 < m.n[0] ? U[sx] : -v, xm = x > 0 ? before : -v;
+        const T ym = ym_in ? U[-sy] : -v, yp = yp_in ? U[sy] : -v;
+        const T zm = zm_in ? U[-1] : -v, zp = zp_in ? U[1] : -v;
+        const T dx = xm - T(2) * v + xp, dy = ym - T(2) * v + yp, dz = zm - T(2) * v + zp;
+        T lap = ihx2 != T(0) ? dx * ihx2 : dx / hx2;
+        lap = lap + (ihy2 != T(0) ? dy * ihy2 : dy / hy2);
+        lap = lap + (ihz2 != T(0) ? dz * ihz2 : dz / hz2);
+        T value = v + (R[0] - v + alpha * lap) / D[0];
+        if (wall || (m.c == 0 && (x == 0 || x + 1 == m.n[0]))) value = T(0);
+        O[0] = value;
+        before = v;
+        v = xp;
+        U += sx;
+        R += sx;
+        D += sx;
+        O += sx;
+    }
 }
 
 // Fixed-order block sums of K values per thread; thread 0 writes them.
@@ -318,8 +355,20 @@ ConstFaces<T> cfaces(const void* const* f) {
 
 bool all3(const void* const* f) { return f && f[0] && f[1] && f[2]; }
 
-int64_t face_total(const Cells& g) {
-    return (g.nx + 1) * g.ny * g.nz + g.nx * (g.ny + 1) * g.nz + g.nx * g.ny * (g.nz + 1);
+// Blocks of 256 columns of the largest face plane, and x chunks so that about
+// 8 blocks per SM of a B200 run, each over as many planes as that leaves.
+dim3 march_grid(const Cells& g, int* chunks) {
+    const int64_t plane = std::max(std::max((g.ny + 1) * g.nz, g.ny * (g.nz + 1)), g.ny * g.nz);
+    const int64_t bx = (plane + 255) / 256, most = std::max<int64_t>(1, 148 * 8 / (3 * bx));
+    *chunks = int(std::min<int64_t>(most, g.nx + 1));
+    return dim3(unsigned(bx), unsigned(3 * *chunks));
+}
+
+// 1/v where v is a power of two whose inverse is normal, else 0.
+template <class T>
+T power_of_two_inverse(T v) {
+    int ex = 0;
+    return v > T(0) && std::isnormal(v) && std::frexp(double(v), &ex) == 0.5 && std::isnormal(T(1) / v) ? T(1) / v : T(0);
 }
 
 unsigned cell_blocks(const Cells& g) { return unsigned((g.nx * g.ny * g.nz + kCells - 1) / kCells); }
@@ -342,13 +391,14 @@ extern "C" int32_t afsi_b200_helmholtz_initialize(const void* const* b, const vo
     AFSI_REQUIRE(all3(b) && all3(diag) && all3(reinterpret_cast<const void* const*>(rhs)) &&
                      all3(reinterpret_cast<const void* const*>(u)) && param && spacing,
                  "null Helmholtz argument");
-    const int64_t total = face_total(g);
+    int chunks = 1;
+    const dim3 grid = march_grid(g, &chunks);
     AFSI_DISPATCH(dtype, {
-        helmholtz_initialize_kernel<T><<<blocks_for(total, 256), 256, 0, stream>>>(
-            cfaces<T>(b), static_cast<const T*>(p), cfaces<T>(diag), faces<T>(rhs), faces<T>(u),
-            static_cast<const T*>(param), g, spacing[0], spacing[1], spacing[2], total);
+        return launch_pdl("helmholtz initialize", helmholtz_initialize_kernel<T>, grid, dim3(256), 0, stream, cfaces<T>(b),
+                          static_cast<const T*>(p), cfaces<T>(diag), faces<T>(rhs), faces<T>(u),
+                          static_cast<const T*>(param), g, spacing[0], spacing[1], spacing[2], chunks);
     });
-    return launched("helmholtz initialize");
+    return AFSI_OK;
 }
 
 extern "C" int32_t afsi_b200_helmholtz_sweep(const void* const* u, const void* const* rhs, const void* const* diag,
@@ -360,13 +410,16 @@ extern "C" int32_t afsi_b200_helmholtz_sweep(const void* const* u, const void* c
     AFSI_REQUIRE(all3(u) && all3(rhs) && all3(diag) && all3(reinterpret_cast<const void* const*>(out)) && param &&
                      spacing_squared,
                  "null Helmholtz argument");
-    const int64_t total = face_total(g);
+    int chunks = 1;
+    const dim3 grid = march_grid(g, &chunks);
     AFSI_DISPATCH(dtype, {
-        helmholtz_sweep_kernel<T><<<blocks_for(total, 256), 256, 0, stream>>>(
-            cfaces<T>(u), cfaces<T>(rhs), cfaces<T>(diag), faces<T>(out), static_cast<const T*>(param), g,
-            spacing_squared[0], spacing_squared[1], spacing_squared[2], total);
+        const T h2[3] = {T(spacing_squared[0]), T(spacing_squared[1]), T(spacing_squared[2])};
+        return launch_pdl("helmholtz sweep", helmholtz_sweep_kernel<T>, grid, dim3(256), 0, stream, cfaces<T>(u),
+                          cfaces<T>(rhs), cfaces<T>(diag), faces<T>(out), static_cast<const T*>(param), g, h2[0], h2[1],
+                          h2[2], power_of_two_inverse(h2[0]), power_of_two_inverse(h2[1]), power_of_two_inverse(h2[2]),
+                          chunks);
     });
-    return launched("helmholtz sweep");
+    return AFSI_OK;
 }
 
 extern "C" int32_t afsi_b200_stokes_start_partial(const void* const* b, const void* p, void* out,

@@ -18,8 +18,10 @@ This module keeps that method, its tolerances and its acceptance test:
 * ``gmres(action, rhs, precondition=..., options=...)`` restates the reference's
   GMRES (two classical Gram-Schmidt passes, Givens estimate with periodic true
   residual checks, restart from the measured residual when an estimate is
-  rejected).  The small Hessenberg system lives on the host; one host read of
-  its new column per iteration (the reference reads it too).
+  rejected).  The Gram-Schmidt passes run in four fused launches
+  (``afsi_b200_krylov_step``).  The small Hessenberg system lives on the host;
+  one host read of its new column per iteration (the reference reads it too),
+  after which the preconditioner's multigrid solve is read as well.
 
 Precision form (``precision='fp32-preconditioner'``): the preconditioner's
 Helmholtz sweeps and V-cycles run in FP32 (FP64 coarsest solve), while the
@@ -77,10 +79,33 @@ class KrylovSpace:
         return self.V, self.Z
 
 
+class _Arnoldi:
+    """The two Gram-Schmidt passes, norms and the new basis row of one GMRES
+    step on the device (``afsi_b200_krylov_step``), over the rows of V."""
+    MOST = 1023
+
+    def __init__(self, V):
+        rows, self.n = V.shape
+        self.V = V
+        self.work = torch.empty(self.n, device=V.device, dtype=V.dtype)
+        self.column = torch.empty(rows + 1, device=V.device, dtype=torch.float64)
+        nbytes = _lib.load().afsi_b200_krylov_scratch_bytes(rows)
+        self.scratch = torch.empty(int(nbytes), device=V.device, dtype=torch.uint8)
+
+    def step(self, j, w):
+        """w against V[:j+1]; V[j+1] set; the Hessenberg column and ||w|| (host)."""
+        w = w.contiguous()
+        call('afsi_b200_krylov_step', ptr(self.V), self.n, j + 1, ptr(w), ptr(self.work), ptr(self.column),
+             ptr(self.scratch), self.scratch.numel(), dtype_code(w.dtype), stream(w.device))
+        return self.column[:j + 3].tolist()
+
+
 @torch.no_grad()
-def gmres(action, rhs, *, precondition=None, options=None, workspace=None):
+def gmres(action, rhs, *, precondition=None, options=None, workspace=None, settle=None):
     """Restarted right-preconditioned GMRES from zero (``nonlinear.py:139-240``);
-    residuals use the original operator; returns (x, info)."""
+    residuals use the original operator; returns (x, info).  settle(), if given,
+    is called after each step's host read, for work that the preconditioner
+    left to be read then."""
     opt = GMRESOptions() if options is None else options
     if rhs.dtype not in (torch.float32, torch.float64) or not rhs.numel():
         raise ValueError('nonempty floating rhs required')
@@ -121,7 +146,8 @@ def gmres(action, rhs, *, precondition=None, options=None, workspace=None):
         else:
             V, Z = workspace.vectors(b, width)
         H = np.zeros((width + 1, width))
-        Hd = b.new_zeros((width + 1, width))
+        arnoldi = _Arnoldi(V) if b.is_cuda and width <= _Arnoldi.MOST else None
+        Hd = b.new_zeros((width + 1, width)) if arnoldi is None else None
         estimated = opt.check_policy == 'estimated'
         rotated = np.zeros((width + 1, width))
         cos, sin = np.zeros(width), np.zeros(width)
@@ -132,16 +158,21 @@ def gmres(action, rhs, *, precondition=None, options=None, workspace=None):
         for j in range(width):
             Z[j] = solve_pre(V[j])
             w = apply(Z[j])
-            original = torch.linalg.vector_norm(w)
-            for _ in range(2):  # classical Gram-Schmidt, twice
-                coefficients = torch.mv(V[:j + 1], w)
-                Hd[:j + 1, j] += coefficients
-                w = w - torch.mv(V[:j + 1].t(), coefficients)
-            Hd[j + 1, j] = torch.linalg.vector_norm(w)
-            column = torch.cat((Hd[:j + 2, j], original.reshape(1))).tolist()  # one host read
+            if arnoldi is not None:
+                column = arnoldi.step(j, w)  # one host read
+            else:
+                original = torch.linalg.vector_norm(w)
+                for _ in range(2):  # classical Gram-Schmidt, twice
+                    coefficients = torch.mv(V[:j + 1], w)
+                    Hd[:j + 1, j] += coefficients
+                    w = w - torch.mv(V[:j + 1].t(), coefficients)
+                Hd[j + 1, j] = torch.linalg.vector_norm(w)
+                column = torch.cat((Hd[:j + 2, j], original.reshape(1))).tolist()  # one host read
+            if settle is not None:
+                settle()
             H[:j + 2, j] = column[:j + 2]
             breakdown = H[j + 1, j] <= 100 * eps * max(column[-1], tiny)
-            if not breakdown:
+            if not breakdown and arnoldi is None:
                 V[j + 1] = w / Hd[j + 1, j]
             count += 1
             converged_estimate = False
@@ -285,12 +316,18 @@ class CNStokes:
 
 
 def _precondition(flow, v, h):
+    """``_precondition_deferred`` with the multigrid solve read: (vector, cycles)."""
+    out, cycles = _precondition_deferred(flow, v, h)
+    return out, cycles()
+
+
+def _precondition_deferred(flow, v, h):
     """pack(t - G phi, (phi + alpha rhs)/h - mean) for t = Helmholtz(r),
     rhs = (-s)/h - D t - mean, phi = multigrid solve of rhs to the
     preconditioner tolerance (``mac/stokes_fgmres.py:46-63``)."""
     work = v if flow.precision == 'fp64' else v.float()
     r, s = flow.unpack(work)
-    tentative = flow.helmholtz.solve(r, out=None)
+    tentative = flow.helmholtz.solve(r, out=flow.helmholtz.result)  # in place: read by this call's kernels only
     st = stream(v.device)
     code = dtype_code(work.dtype)
     rhs = torch.empty(flow.grid.shape, device=v.device, dtype=work.dtype)
@@ -298,13 +335,21 @@ def _precondition(flow, v, h):
     call('afsi_b200_stokes_precondition_rhs', tp, ptr(s), ptr(rhs), ptr(flow.sums), ptr(flow.scratch), flow._shape,
          flow._spacing, h, code, st)
     call('afsi_b200_subtract_mean', ptr(rhs), rhs.numel(), ptr(flow.sums), code, st)
-    phi, info = flow.pressure_solver.solve(rhs, rtol=flow.preconditioner_rtol)
+    # The solve's host read waits until the step's own (the returned reader): its
+    # device loop always runs to the end when check blocks divide max_cycles.
+    opt = flow.pressure_solver.options
+    if opt.max_cycles % opt.check_every == 0:
+        pending = flow.pressure_solver.solve_deferred(rhs, rtol=flow.preconditioner_rtol)
+        phi, cycles = pending.p, lambda: pending.result()[1]['cycles']
+    else:
+        phi, info = flow.pressure_solver.solve(rhs, rtol=flow.preconditioner_rtol)
+        cycles = lambda: info['cycles']
     out = torch.empty(flow.size, device=v.device, dtype=work.dtype)
     call('afsi_b200_stokes_precondition_result', tp, ptr(phi), ptr(rhs), ptr(out), ptr(flow.sums[1:]),
          ptr(flow.scratch), flow._shape, flow._spacing, flow.alpha, h, code, st)
     q = out[flow.faces:]
     call('afsi_b200_subtract_mean', ptr(q), q.numel(), ptr(flow.sums[1:]), code, st)
-    return (out if flow.precision == 'fp64' else out.double()), info['cycles']
+    return (out if flow.precision == 'fp64' else out.double()), cycles
 
 
 def ctypes_ptrs(faces):
@@ -347,11 +392,17 @@ def solve(flow, b, initial=None):
 
     counters = dict(poisson_solves=0, cycles=0)
 
+    unread = []
+
     def precondition(v):
-        out, cycles = _precondition(flow, v.contiguous(), h)
+        out, cycles = _precondition_deferred(flow, v.contiguous(), h)
         counters['poisson_solves'] += 1
-        counters['cycles'] += cycles
+        unread.append(cycles)
         return out
+
+    def settle():
+        while unread:
+            counters['cycles'] += unread.pop()()
 
     norm_b = torch.sqrt(sum(v.square().sum() for v in b)).item()
     if not isfinite(norm_b):
@@ -376,7 +427,8 @@ def solve(flow, b, initial=None):
     tolerance = .5 * min(momentum_tol, h * div_tol)
     controls = GMRESOptions(rtol=0., atol=tolerance, restart=flow.restart, max_iterations=flow.max_iterations,
                             check_policy='estimated', true_check_interval=5)
-    correction, info = gmres(action, rhs, precondition=precondition, options=controls, workspace=flow.krylov)
+    correction, info = gmres(action, rhs, precondition=precondition, options=controls, workspace=flow.krylov,
+                             settle=settle)
     u, q = flow.unpack(guess + correction)
     p = h / scale * (q - q.mean())
     u = tuple(t.contiguous() for t in u)

@@ -730,6 +730,16 @@ int32_t afsi_b200_stokes_precondition_result(const void* const* tentative, const
     void* out, double* sum_out, void* scratch, const int64_t* shape, const double* spacing, double alpha,
     double h, int32_t dtype, afsi_stream_t stream);
 
+/* One Arnoldi step of the flexible GMRES (nonlinear.py:139-240): w (n values,
+ * not written) against rows 0..k-1 of V (row-major, n per row) by classical
+ * Gram-Schmidt taken twice, then V[k] = w''/||w''||.  work: n values; column
+ * (device double[k + 2]): the k coefficients, ||w''||, ||w||.  scratch:
+ * afsi_b200_krylov_scratch_bytes(rows of V) device bytes, rows <= 1024. */
+int64_t afsi_b200_krylov_scratch_bytes(int64_t rows);
+int32_t afsi_b200_krylov_step(void* V, int64_t n, int64_t k, const void* w, void* work, double* column,
+    void* scratch, int64_t scratch_bytes, int32_t dtype, afsi_stream_t stream);
+
+
 /* ---- batched 2D transfers (the batching form) ------------------------------
  * Many independent 2D channel instances (TriangleTransfer, mac2d/transfer.py:
  * 61-127, one per instance in the reference) in one launch per operation.
