@@ -26,10 +26,9 @@
 // changes in how it is executed, none in what is computed:
 //  * the mean-zero gauge (p -= mean after each smoothing block, rhs -= mean
 //    after restriction) is carried as a pending shift: the kernel that writes
-//    a field also reduces its sum (deterministic per-block partials, summed
-//    in index order by the last block to finish), and the next kernel that
-//    reads the field subtracts sum/n on load, so no separate mean or subtract
-//    launches exist;
+//    a field leaves one partial sum per block, and the next kernel that reads
+//    the field adds the partials in a fixed order (pending_mean) and subtracts
+//    sum/n on load, so no separate mean or subtract launches exist;
 //  * zeroing the coarse iterate is folded into the first sweep (p_in = 0);
 //  * every level with at most kCoarseCells cells, the dense coarsest solve
 //    included, runs inside one thread block in shared memory.
@@ -53,8 +52,8 @@ namespace afsi {
 // predecessor (the single-CTA coarse levels use the same update).
 template <int BC, bool Exact, class T>
 __global__ void __launch_bounds__(kThreads) sweep_kernel(const T* __restrict__ p, T* __restrict__ rhs, T* __restrict__ out,
-                                                         Lv<T> L, const double* p_sum, const double* rhs_sum,
-                                                         Site emit, int fix_rhs, int do_emit) {
+                                                         Lv<T> L, Pending p_sum, Pending rhs_sum, Site emit,
+                                                         int fix_rhs, int do_emit) {
     __shared__ T wtab[64];
     if (!Exact) {
         const unsigned t = thread_linear();
@@ -63,8 +62,8 @@ __global__ void __launch_bounds__(kThreads) sweep_kernel(const T* __restrict__ p
     }
     pdl_enter();
     double local = 0.0;
-    const T m = T(site_mean(p_sum, L.n));
-    const T mr = T(site_mean(rhs_sum, L.n));
+    const T m = T(pending_mean(p_sum, L.n));
+    const T mr = T(pending_mean(rhs_sum, L.n));
     for_my_cells<BC>(L, [&](int x, int y, int z) {
         const int64_t i = index_of(x, y, z, L);
         T r = rhs[i];
@@ -93,154 +92,202 @@ __global__ void __launch_bounds__(kThreads) sweep_kernel(const T* __restrict__ p
         out[i] = v;
         local += double(v);
     });
-    if (do_emit) site_finish(emit, local);
+    if (do_emit) site_put(emit, local);
 }
 
-// (A p) of the z-adjacent cells (x,y,z) and (x,y,z+1), z even, of a 3D
-// level (Neumann or Dirichlet), every load shifted by m: neg_lap's fast-form
-// terms in neg_lap's order for each cell, with the pair and its x and y
-// neighbours read as 16-byte vectors and the two outer z neighbours as
-// scalars.  Returns the shifted centre values in pc0, pc1.
+// Two z-adjacent values.
+template <class T>
+using ZPair = typename std::conditional<sizeof(T) == 8, double2, float2>::type;
+
+template <class T>
+__device__ __forceinline__ ZPair<T> load_pair(const T* p, T m = T(0)) {
+    ZPair<T> v = *reinterpret_cast<const ZPair<T>*>(p);
+    v.x = v.x - m;
+    v.y = v.y - m;
+    return v;
+}
+
+// Which neighbours of a z pair exist.
+struct PairSides {
+    bool xp, xm, yp, ym, zp, zm;
+};
+
+// (A p) of the z-adjacent cells (x,y,z) and (x,y,z+1), z even, of a 3D level
+// (Neumann or Dirichlet) from the pair c, its x and y neighbour pairs and the
+// outer z neighbours zm, zq: neg_lap's fast-form terms in neg_lap's order for
+// each cell.  Values of sides that do not exist are not used.
 template <int BC, class T>
-__device__ __forceinline__ void pair_neg_lap(const T* __restrict__ p, int64_t i, int x, int y, int z, const Lv<T>& L,
-                                             T m, T& pc0, T& pc1, T& a0, T& a1) {
-    using V = typename std::conditional<sizeof(T) == 8, double2, float2>::type;
-    const int64_t sx = int64_t(L.ny) * L.nz, sy = L.nz;
-    const bool xp_in = x + 1 < L.nx, xm_in = x > 0, yp_in = y + 1 < L.ny, ym_in = y > 0, zm_in = z > 0,
-               zp_in = z + 2 < L.nz;
-    const V c = *reinterpret_cast<const V*>(p + i);
-    pc0 = c.x - m;
-    pc1 = c.y - m;
-    V xp, xm, yp, ym;
-    if (xp_in) xp = *reinterpret_cast<const V*>(p + i + sx);
-    if (xm_in) xm = *reinterpret_cast<const V*>(p + i - sx);
-    if (yp_in) yp = *reinterpret_cast<const V*>(p + i + sy);
-    if (ym_in) ym = *reinterpret_cast<const V*>(p + i - sy);
-    const T zm = zm_in ? p[i - 1] - m : T(0), zq = zp_in ? p[i + 2] - m : T(0);
+__device__ __forceinline__ void pair_neg_lap(const ZPair<T>& c, const ZPair<T>& xp, const ZPair<T>& xm,
+                                             const ZPair<T>& yp, const ZPair<T>& ym, T zm, T zq, const PairSides& in,
+                                             const Lv<T>& L, T& a0, T& a1) {
+    const T pc0 = c.x, pc1 = c.y;
     a0 = T(0);
     a1 = T(0);
     if (BC == AFSI_BC_DIRICHLET) {
-        a0 = xp_in ? a0 - ((xp.x - m) - pc0) * L.ih2[0] : a0 + (pc0 + pc0) * L.ih2[0];
-        a1 = xp_in ? a1 - ((xp.y - m) - pc1) * L.ih2[0] : a1 + (pc1 + pc1) * L.ih2[0];
-        a0 = xm_in ? a0 + (pc0 - (xm.x - m)) * L.ih2[0] : a0 + (pc0 + pc0) * L.ih2[0];
-        a1 = xm_in ? a1 + (pc1 - (xm.y - m)) * L.ih2[0] : a1 + (pc1 + pc1) * L.ih2[0];
-        a0 = yp_in ? a0 - ((yp.x - m) - pc0) * L.ih2[1] : a0 + (pc0 + pc0) * L.ih2[1];
-        a1 = yp_in ? a1 - ((yp.y - m) - pc1) * L.ih2[1] : a1 + (pc1 + pc1) * L.ih2[1];
-        a0 = ym_in ? a0 + (pc0 - (ym.x - m)) * L.ih2[1] : a0 + (pc0 + pc0) * L.ih2[1];
-        a1 = ym_in ? a1 + (pc1 - (ym.y - m)) * L.ih2[1] : a1 + (pc1 + pc1) * L.ih2[1];
+        a0 = in.xp ? a0 - (xp.x - pc0) * L.ih2[0] : a0 + (pc0 + pc0) * L.ih2[0];
+        a1 = in.xp ? a1 - (xp.y - pc1) * L.ih2[0] : a1 + (pc1 + pc1) * L.ih2[0];
+        a0 = in.xm ? a0 + (pc0 - xm.x) * L.ih2[0] : a0 + (pc0 + pc0) * L.ih2[0];
+        a1 = in.xm ? a1 + (pc1 - xm.y) * L.ih2[0] : a1 + (pc1 + pc1) * L.ih2[0];
+        a0 = in.yp ? a0 - (yp.x - pc0) * L.ih2[1] : a0 + (pc0 + pc0) * L.ih2[1];
+        a1 = in.yp ? a1 - (yp.y - pc1) * L.ih2[1] : a1 + (pc1 + pc1) * L.ih2[1];
+        a0 = in.ym ? a0 + (pc0 - ym.x) * L.ih2[1] : a0 + (pc0 + pc0) * L.ih2[1];
+        a1 = in.ym ? a1 + (pc1 - ym.y) * L.ih2[1] : a1 + (pc1 + pc1) * L.ih2[1];
         a0 = a0 - (pc1 - pc0) * L.ih2[2];
-        a1 = zp_in ? a1 - (zq - pc1) * L.ih2[2] : a1 + (pc1 + pc1) * L.ih2[2];
-        a0 = zm_in ? a0 + (pc0 - zm) * L.ih2[2] : a0 + (pc0 + pc0) * L.ih2[2];
+        a1 = in.zp ? a1 - (zq - pc1) * L.ih2[2] : a1 + (pc1 + pc1) * L.ih2[2];
+        a0 = in.zm ? a0 + (pc0 - zm) * L.ih2[2] : a0 + (pc0 + pc0) * L.ih2[2];
         a1 = a1 + (pc1 - pc0) * L.ih2[2];
     } else {
-        if (xp_in) {
-            a0 = a0 - ((xp.x - m) - pc0) * L.ih2[0];
-            a1 = a1 - ((xp.y - m) - pc1) * L.ih2[0];
+        if (in.xp) {
+            a0 = a0 - (xp.x - pc0) * L.ih2[0];
+            a1 = a1 - (xp.y - pc1) * L.ih2[0];
         }
-        if (xm_in) {
-            a0 = a0 + (pc0 - (xm.x - m)) * L.ih2[0];
-            a1 = a1 + (pc1 - (xm.y - m)) * L.ih2[0];
+        if (in.xm) {
+            a0 = a0 + (pc0 - xm.x) * L.ih2[0];
+            a1 = a1 + (pc1 - xm.y) * L.ih2[0];
         }
-        if (yp_in) {
-            a0 = a0 - ((yp.x - m) - pc0) * L.ih2[1];
-            a1 = a1 - ((yp.y - m) - pc1) * L.ih2[1];
+        if (in.yp) {
+            a0 = a0 - (yp.x - pc0) * L.ih2[1];
+            a1 = a1 - (yp.y - pc1) * L.ih2[1];
         }
-        if (ym_in) {
-            a0 = a0 + (pc0 - (ym.x - m)) * L.ih2[1];
-            a1 = a1 + (pc1 - (ym.y - m)) * L.ih2[1];
+        if (in.ym) {
+            a0 = a0 + (pc0 - ym.x) * L.ih2[1];
+            a1 = a1 + (pc1 - ym.y) * L.ih2[1];
         }
         a0 = a0 - (pc1 - pc0) * L.ih2[2];
-        if (zp_in) a1 = a1 - (zq - pc1) * L.ih2[2];
-        if (zm_in) a0 = a0 + (pc0 - zm) * L.ih2[2];
+        if (in.zp) a1 = a1 - (zq - pc1) * L.ih2[2];
+        if (in.zm) a0 = a0 + (pc0 - zm) * L.ih2[2];
         a1 = a1 + (pc1 - pc0) * L.ih2[2];
     }
 }
 
-// The fast-form Jacobi sweep of a 3D level (Neumann or Dirichlet) with two
-// z-adjacent cells per thread, z = 2k and 2k+1 (nz even): the pair's p and
-// rhs and its x and y neighbours are 16-byte loads, the outer z neighbours
-// two 8-byte loads, and the pair shares its address and x/y tests.  No
-// pending shift of p (the launched sweeps take none); fix_rhs subtracts the
-// rhs mean and writes it back.  Per cell the same operations in the same
-// order as sweep_kernel's fast form, so out is bitwise equal; the emitted sum
-// is added per block in this kernel's cell order.
+// The fast-form Jacobi sweep of a 3D level (Neumann or Dirichlet): a thread
+// owns the column of z pairs (y, z = 2k and 2k+1; nz even) and marches
+// `planes` planes along x, keeping the pair before, at and after the plane in
+// registers, so p is read from the L2 once and not three times (a plane per
+// thread read 89 MB per sweep at 128^3, 14 us; now 57 MB, 12 us).  The pair's
+// values and its y neighbours are 16-byte loads, the outer z neighbours two
+// scalars.  No pending shift of p (the launched sweeps take none); fix_rhs
+// subtracts the rhs mean and writes it back.  Per cell the same operations in
+// the same order as sweep_kernel's fast form, so out is bitwise equal; the
+// emitted sum is added per block in this kernel's cell order.
 template <int BC, class T>
-__global__ void __launch_bounds__(kThreads) sweep_zpair_kernel(const T* __restrict__ p, T* __restrict__ rhs,
-                                                               T* __restrict__ out, Lv<T> L, const double* rhs_sum,
-                                                               Site emit, int fix_rhs, int do_emit) {
-    using V = typename std::conditional<sizeof(T) == 8, double2, float2>::type;
+__global__ void __launch_bounds__(kThreads, 4) sweep_columns_kernel(const T* __restrict__ p, T* __restrict__ rhs,
+                                                                    T* __restrict__ out, Lv<T> L, Pending rhs_sum,
+                                                                    Site emit, int planes, int fix_rhs, int do_emit) {
+    using V = ZPair<T>;
     __shared__ T wtab[64];
     {
         const unsigned t = thread_linear();
         if (t < 64) wtab[t] = omega_of_class<BC>(int(t), L);
         __syncthreads();
     }
+    const int y = blockIdx.y * blockDim.y + threadIdx.y, z = 2 * int(blockIdx.x * blockDim.x + threadIdx.x);
+    const int x0 = int(blockIdx.z) * planes, x1 = min(x0 + planes, L.nx);
     pdl_enter();
     double local = 0.0;
-    const T mr = T(site_mean(rhs_sum, L.n));
-    const int zp = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
-    const int z = 2 * zp;
-    if (z < L.nz && y < L.ny) {
-        for (int x = blockIdx.z; x < L.nx; x += gridDim.z) {
-            const int64_t i = (int64_t(x) * L.ny + y) * L.nz + z;
-            const V rv = *reinterpret_cast<const V*>(rhs + i);
-            T r0 = rv.x, r1 = rv.y;
-            if (fix_rhs) {
-                r0 = r0 - mr;
-                r1 = r1 - mr;
-                V w;
-                w.x = r0;
-                w.y = r1;
-                *reinterpret_cast<V*>(rhs + i) = w;
-            }
-            const T w0 = wtab[boundary_class(x, y, z, L.nx, L.ny, L.nz)];
-            const T w1 = wtab[boundary_class(x, y, z + 1, L.nx, L.ny, L.nz)];
-            T v0, v1;
+    const T mr = fix_rhs ? T(pending_mean(rhs_sum, L.n)) : T(0);
+    if (z < L.nz && y < L.ny && x0 < x1) {
+        const int64_t sx = int64_t(L.ny) * L.nz, sy = L.nz;
+        int64_t i = (int64_t(x0) * L.ny + y) * L.nz + z;
+        PairSides in;
+        in.yp = y + 1 < L.ny;
+        in.ym = y > 0;
+        in.zp = z + 2 < L.nz;
+        in.zm = z > 0;
+        // x = 1 of a level of more than two planes: no x bit set
+        const int c0 = boundary_class(1, y, z, 1 << 30, L.ny, L.nz), c1 = boundary_class(1, y, z + 1, 1 << 30, L.ny, L.nz);
+        V c = {}, before = {};
+        if (p) {
+            c = load_pair(p + i);
+            if (x0 > 0) before = load_pair(p + i - sx);
+        }
+        for (int x = x0; x < x1; ++x, i += sx) {
+            in.xp = x + 1 < L.nx;
+            in.xm = x > 0;
+            V r = load_pair(rhs + i);
+            V after = {}, yp = {}, ym = {};
+            T zm = T(0), zq = T(0);
             if (p) {
-                T pc0, pc1, a0, a1;
-                pair_neg_lap<BC>(p, i, x, y, z, L, T(0), pc0, pc1, a0, a1);
-                v0 = jacobi_update(pc0, r0, a0, w0);
-                v1 = jacobi_update(pc1, r1, a1, w1);
-            } else {
-                v0 = r0 * w0;
-                v1 = r1 * w1;
+                if (in.xp) after = load_pair(p + i + sx);
+                if (in.yp) yp = load_pair(p + i + sy);
+                if (in.ym) ym = load_pair(p + i - sy);
+                if (in.zm) zm = p[i - 1];
+                if (in.zp) zq = p[i + 2];
             }
+            if (fix_rhs) {
+                r.x = r.x - mr;
+                r.y = r.y - mr;
+                *reinterpret_cast<V*>(rhs + i) = r;
+            }
+            const int cx = (x == 0) | ((x == L.nx - 1) << 1);
+            const T w0 = wtab[c0 | cx], w1 = wtab[c1 | cx];
             V o;
-            o.x = v0;
-            o.y = v1;
+            if (p) {
+                T a0, a1;
+                pair_neg_lap<BC>(c, after, before, yp, ym, zm, zq, in, L, a0, a1);
+                o.x = jacobi_update(c.x, r.x, a0, w0);
+                o.y = jacobi_update(c.y, r.y, a1, w1);
+            } else {
+                o.x = r.x * w0;
+                o.y = r.y * w1;
+            }
             *reinterpret_cast<V*>(out + i) = o;
-            local += double(v0);
-            local += double(v1);
+            local += double(o.x);
+            local += double(o.y);
+            before = c;
+            c = after;
         }
     }
-    if (do_emit) site_finish(emit, local);
+    if (do_emit) site_put(emit, local);
 }
 
 // residual_restrict_kernel's fast form for 3D levels (Neumann or Dirichlet)
-// with the fine z pairs of each coarse cell read by pair_neg_lap: the eight
-// children summed in the same order (x, y, then z), so coarse is bitwise
-// equal.
+// with the fine z pairs of each coarse cell read as 16-byte vectors, each once
+// (the four pairs are each other's x and y neighbours): the eight children
+// summed in the same order (x, y, then z), so coarse is bitwise equal.
 template <int BC, class T>
 __global__ void __launch_bounds__(kThreads) residual_restrict_zpair_kernel(const T* __restrict__ p,
                                                                           const T* __restrict__ rhs,
                                                                           T* __restrict__ coarse, Lv<T> L, Lv<T> C,
-                                                                          const double* p_sum, Site emit,
-                                                                          int do_emit) {
-    using V = typename std::conditional<sizeof(T) == 8, double2, float2>::type;
+                                                                          Pending p_sum, Site emit, int do_emit) {
+    using V = ZPair<T>;
     pdl_enter();
     double local = 0.0;
-    const T m = T(site_mean(p_sum, L.n));
+    const T m = T(pending_mean(p_sum, L.n));
+    const int64_t sx = int64_t(L.ny) * L.nz, sy = L.nz;
     for_my_cells<BC>(C, [&](int cx, int cy, int cz) {
+        const int64_t i = index_of(2 * cx, 2 * cy, 2 * cz, L);
+        const bool xm_in = cx > 0, xp_in = cx + 1 < C.nx, ym_in = cy > 0, yp_in = cy + 1 < C.ny;
+        V c[2][2], xo[2][2] = {}, yo[2][2] = {};  // pairs; outer x neighbours [side][b]; outer y neighbours [a][side]
+#pragma unroll
+        for (int a = 0; a < 2; ++a)
+#pragma unroll
+            for (int b = 0; b < 2; ++b) c[a][b] = load_pair(p + i + a * sx + b * sy, m);
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            if (xm_in) xo[0][k] = load_pair(p + i - sx + k * sy, m);
+            if (xp_in) xo[1][k] = load_pair(p + i + 2 * sx + k * sy, m);
+            if (ym_in) yo[k][0] = load_pair(p + i - sy + k * sx, m);
+            if (yp_in) yo[k][1] = load_pair(p + i + 2 * sy + k * sx, m);
+        }
+        PairSides in;
+        in.zm = cz > 0;
+        in.zp = cz + 1 < C.nz;
         T v = T(0);
 #pragma unroll
         for (int a = 0; a < 2; ++a)
 #pragma unroll
             for (int b = 0; b < 2; ++b) {
-                const int x = 2 * cx + a, y = 2 * cy + b, z = 2 * cz;
-                const int64_t i = index_of(x, y, z, L);
-                T pc0, pc1, a0, a1;
-                pair_neg_lap<BC>(p, i, x, y, z, L, m, pc0, pc1, a0, a1);
-                const V r = *reinterpret_cast<const V*>(rhs + i);
+                const int64_t j = i + a * sx + b * sy;
+                const T zm = in.zm ? p[j - 1] - m : T(0), zq = in.zp ? p[j + 2] - m : T(0);
+                in.xm = a == 1 || xm_in;
+                in.xp = a == 0 || xp_in;
+                in.ym = b == 1 || ym_in;
+                in.yp = b == 0 || yp_in;
+                T a0, a1;
+                pair_neg_lap<BC>(c[a][b], a == 0 ? c[1][b] : xo[1][b], a == 0 ? xo[0][b] : c[0][b],
+                                 b == 0 ? c[a][1] : yo[a][1], b == 0 ? yo[a][0] : c[a][0], zm, zq, in, L, a0, a1);
+                const V r = load_pair(rhs + j);
                 v = v + (r.x - a0);
                 v = v + (r.y - a1);
             }
@@ -248,7 +295,7 @@ __global__ void __launch_bounds__(kThreads) residual_restrict_zpair_kernel(const
         coarse[index_of(cx, cy, cz, C)] = v;
         local += double(v);
     });
-    if (do_emit) site_finish(emit, local);
+    if (do_emit) site_put(emit, local);
 }
 
 // coarse[c] = mean of children of (rhs - A p), p shifted by m_p.  Launched
@@ -256,27 +303,83 @@ __global__ void __launch_bounds__(kThreads) residual_restrict_zpair_kernel(const
 template <int BC, bool Exact, class T>
 __global__ void __launch_bounds__(kThreads) residual_restrict_kernel(const T* __restrict__ p, const T* __restrict__ rhs,
                                                                      T* __restrict__ coarse, Lv<T> L, Lv<T> C,
-                                                                     const double* p_sum, Site emit, int do_emit) {
+                                                                     Pending p_sum, Site emit, int do_emit) {
     pdl_enter();
     double local = 0.0;
-    const T m = T(site_mean(p_sum, L.n));
+    const T m = T(pending_mean(p_sum, L.n));
     for_my_cells<BC>(C, [&](int cx, int cy, int cz) {
         const T v = restrict_residual_at<BC, Exact>(p, rhs, cx, cy, cz, L, m);
         coarse[index_of(cx, cy, cz, C)] = v;
         local += double(v);
     });
-    if (do_emit) site_finish(emit, local);
+    if (do_emit) site_put(emit, local);
 }
 
 // dst = (src - m_src) + P(corr - m_corr); src may alias dst (own cell only).
 template <int BC, class T>
 __global__ void __launch_bounds__(kThreads) prolong_kernel(const T* src, const T* __restrict__ corr, T* dst, Lv<T> L,
-                                                           Lv<T> C, const double* src_sum, const double* corr_sum) {
+                                                           Lv<T> C, Pending src_sum, Pending corr_sum) {
     pdl_enter();
-    const T ms = T(site_mean(src_sum, L.n)), mc = T(site_mean(corr_sum, C.n));
+    const T ms = T(pending_mean(src_sum, L.n)), mc = T(pending_mean(corr_sum, C.n));
     for_my_cells<BC>(L, [&](int x, int y, int z) {
         const int64_t i = index_of(x, y, z, L);
         dst[i] = (src[i] - ms) + prolong_at<BC>(corr, x, y, z, C, mc);
+    });
+}
+
+// prolong_kernel for 3D levels, a thread per coarse cell: the eight fine
+// cells of a coarse cell draw on its 3x3x3 neighbourhood, so 27 loads and the
+// z and y interpolations they share serve eight cells (64 loads in
+// prolong_kernel).  Fine values are read and written as z pairs.  The same
+// interpolations in the same order per cell (z, then y, then x): bitwise equal.
+template <int BC, class T>
+__global__ void __launch_bounds__(kThreads) prolong_octet_kernel(const T* src, const T* __restrict__ corr, T* dst,
+                                                                 Lv<T> L, Lv<T> C, Pending src_sum, Pending corr_sum) {
+    using V = ZPair<T>;
+    pdl_enter();
+    const T ms = T(pending_mean(src_sum, L.n)), mc = T(pending_mean(corr_sum, C.n));
+    const bool odd = BC == AFSI_BC_DIRICHLET;  // ghosts are negated edge values (odd extension)
+    const T near_ = T(.75), far_ = T(.25);
+    for_my_cells<BC>(C, [&](int cx, int cy, int cz) {
+        const int zs[3] = {cz > 0 ? cz - 1 : 0, cz, cz + 1 < C.nz ? cz + 1 : cz};
+        const bool gz[3] = {odd && cz == 0, false, odd && cz + 1 == C.nz};
+        T row[3][2][2];  // [x neighbour][fine y parity][fine z parity]
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            const int x = i == 0 ? (cx > 0 ? cx - 1 : 0) : i == 1 ? cx : (cx + 1 < C.nx ? cx + 1 : cx);
+            const bool gx = odd && ((i == 0 && cx == 0) || (i == 2 && cx + 1 == C.nx));
+            T lz[3][2];
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+                const int y = j == 0 ? (cy > 0 ? cy - 1 : 0) : j == 1 ? cy : (cy + 1 < C.ny ? cy + 1 : cy);
+                const bool gy = odd && ((j == 0 && cy == 0) || (j == 2 && cy + 1 == C.ny));
+                const T* line = corr + (int64_t(x) * C.ny + y) * C.nz;
+                T v[3];
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    v[k] = line[zs[k]] - mc;
+                    if ((gx != gy) != gz[k]) v[k] = -v[k];  // one sign flip per ghost axis
+                }
+                lz[j][0] = v[0] * far_ + v[1] * near_;
+                lz[j][1] = v[1] * near_ + v[2] * far_;
+            }
+#pragma unroll
+            for (int d = 0; d < 2; ++d) {
+                row[i][0][d] = lz[0][d] * far_ + lz[1][d] * near_;
+                row[i][1][d] = lz[1][d] * near_ + lz[2][d] * far_;
+            }
+        }
+#pragma unroll
+        for (int a = 0; a < 2; ++a)
+#pragma unroll
+            for (int b = 0; b < 2; ++b) {
+                const int64_t i = index_of(2 * cx + a, 2 * cy + b, 2 * cz, L);
+                const V s = load_pair(src + i, ms);
+                V o;
+                o.x = s.x + (row[a][b][0] * (a ? near_ : far_) + row[a + 1][b][0] * (a ? far_ : near_));
+                o.y = s.y + (row[a][b][1] * (a ? near_ : far_) + row[a + 1][b][1] * (a ? far_ : near_));
+                *reinterpret_cast<V*>(dst + i) = o;
+            }
     });
 }
 
@@ -288,11 +391,11 @@ __global__ void __launch_bounds__(kThreads) prolong_kernel(const T* src, const T
 // same) and, in the last block, the loop decision of mg_decide_kernel.
 template <int BC, class T>
 __global__ void __launch_bounds__(kThreads) finalize_check_kernel(const T* src, T* dst, const T* __restrict__ rhs,
-                                                                  Lv<T> L, const double* sum, Site s, double* norm,
+                                                                  Lv<T> L, Pending sum, Site s, double* norm,
                                                                   double* loop, int check_every, int max_cycles,
                                                                   cudaGraphConditionalHandle handle) {
     pdl_enter();
-    const T m = T(site_mean(sum, L.n));
+    const T m = T(pending_mean(sum, L.n));
     const bool write = src != dst;
     double local = 0.0;
     for_my_cells<BC>(L, [&](int x, int y, int z) {
@@ -315,9 +418,9 @@ __global__ void __launch_bounds__(kThreads) finalize_check_kernel(const T* src, 
 
 // dst = src - sum/n (or a copy when sum is null); flat grid-stride.
 template <class T>
-__global__ void __launch_bounds__(kThreads) shift_kernel(const T* src, T* dst, int64_t n, const double* sum) {
+__global__ void __launch_bounds__(kThreads) shift_kernel(const T* src, T* dst, int64_t n, Pending sum) {
     pdl_enter();
-    const T m = T(site_mean(sum, n));
+    const T m = T(pending_mean(sum, n));
     for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
         dst[i] = src[i] - m;
 }
@@ -415,7 +518,7 @@ __global__ void __launch_bounds__(kThreads) stats_kernel(const T* __restrict__ x
 // (cluster_cycle).
 template <int BC, class T, class TC>
 __global__ void __launch_bounds__(kCoarseThreads) cluster_kernel(const T* __restrict__ rhs_global,
-                                                                const double* rhs_sum, const T* p_global, T* p_out,
+                                                                Pending rhs_sum, const T* p_global, T* p_out,
                                                                 const TC* __restrict__ cinv, ClusterLevels<T> cl,
                                                                 int smooth) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -426,7 +529,7 @@ __global__ void __launch_bounds__(kCoarseThreads) cluster_kernel(const T* __rest
 
 // Levels of one V-cycle from `first` down, in one CTA (coarse_cycle).
 template <int BC, class T, class TC>
-__global__ void __launch_bounds__(kCoarseThreads) coarse_kernel(const T* __restrict__ rhs_global, const double* rhs_sum,
+__global__ void __launch_bounds__(kCoarseThreads) coarse_kernel(const T* __restrict__ rhs_global, Pending rhs_sum,
                                                                const T* p_global, T* p_out, const TC* __restrict__ cinv,
                                                                CoarseLevels<T> cl, int smooth) {
     pdl_enter();
@@ -567,11 +670,19 @@ Geometry launch_for(const Lv<T>& L, int bc) {
     return g;
 }
 
-// Geometry of sweep_zpair_kernel: launch_for with the z extent halved.
+// Geometry of sweep_columns_kernel: launch_for's block over (z pairs, y), and
+// x chunks of `planes` planes so that one wave of blocks (four per SM of a
+// B200) covers the level; a level of fewer blocks takes a plane per chunk.
 template <class T>
-Geometry launch_for_zpairs(Lv<T> L) {
+Geometry launch_for_columns(Lv<T> L, int* planes) {
+    const int nx = L.nx;
     L.nz /= 2;
-    return launch_for(L, AFSI_BC_NEUMANN);
+    Geometry g = launch_for(L, AFSI_BC_NEUMANN);
+    const int most = std::max(1, 592 / int(g.grid.x * g.grid.y));
+    *planes = (nx + most - 1) / most;
+    g.grid.z = (nx + *planes - 1) / *planes;
+    g.blocks = int64_t(g.grid.x) * g.grid.y * g.grid.z;
+    return g;
 }
 
 int flat_grid(int64_t n) {
@@ -706,8 +817,9 @@ struct Runner {
     T* Q(int l) const { return static_cast<T*>(plan->level[l].ping); }
     T* R(int l) const { return static_cast<T*>(plan->level[l].rhs); }
     static constexpr bool singular = singular_bc(BC);
+    static constexpr Pending none{nullptr, 0};
 
-    // Two z cells per thread (sweep_zpair_kernel) on 3D levels with even nz
+    // Two z cells per thread (sweep_columns_kernel) on 3D levels with even nz
     // whose buffers are 16-byte aligned.
     bool zpairs(int l) const {
         if constexpr (BC == AFSI_BC_NEUMANN || BC == AFSI_BC_DIRICHLET) {
@@ -718,7 +830,7 @@ struct Runner {
         }
     }
 
-    int32_t coarse(int l, const double* rhs_sum, T** out) {
+    int32_t coarse(int l, Pending rhs_sum, T** out) {
         CoarseLevels<T> cl;
         for (int k = 0; k < plan->levels; ++k) cl.lv[k] = lv[k];
         cl.first = l;
@@ -737,7 +849,7 @@ struct Runner {
                           cl, plan->smooth);
     }
 
-    int32_t cluster(int l, const double* rhs_sum, T** out) {
+    int32_t cluster(int l, Pending rhs_sum, T** out) {
         *out = P(l);
         if constexpr (is3d(BC)) {
             cudaLaunchConfig_t cfg = {};
@@ -846,92 +958,95 @@ struct Runner {
         return capacity < 0 ? 0 : capacity;
     }
 
-    // Returns the buffer holding the level's final iterate and the site whose
-    // sum is its pending mean (nullptr: exact).
-    int32_t level(int l, T** out, const double** out_sum) {
-        int32_t rc;
-        if (l >= first_cluster) {
-            rc = cluster(l, (l > 0 && singular) ? st.s[l][2].result : nullptr, out);
-            *out_sum = nullptr;
-            return rc;
-        }
-        if (l >= first_coarse) {
-            rc = coarse(l, (l > 0 && singular) ? st.s[l][2].result : nullptr, out);
-            *out_sum = nullptr;
-            return rc;
-        }
+    // One sweep of level l; emit: its block sums go to site k (pending afterwards).
+    int32_t sweep(int l, const T* src, T* dst, Pending rhs_sum, int k, bool emit, Pending* pending) {
         const Lv<T>& L = lv[l];
-        const Geometry g = launch_for(L, BC);
-        const Geometry gz = launch_for_zpairs(L);
+        int64_t blocks;
+        int32_t rc;
+        if (zpairs(l)) {
+            int planes = 1;
+            const Geometry g = launch_for_columns(L, &planes);
+            rc = launch_pdl("mg sweep", sweep_columns_kernel<BC, T>, g.grid, g.block, 0, stream, src, R(l), dst, L, rhs_sum,
+                            st.s[l][k], planes, rhs_sum.part ? 1 : 0, emit ? 1 : 0);
+            blocks = g.blocks;
+        } else {
+            const Geometry g = launch_for(L, BC);
+            rc = launch_pdl("mg sweep", sweep_kernel<BC, false, T>, g.grid, g.block, 0, stream, src, R(l), dst, L, none,
+                            rhs_sum, st.s[l][k], rhs_sum.part ? 1 : 0, emit ? 1 : 0);
+            blocks = g.blocks;
+        }
+        if (emit) *pending = Pending{st.s[l][k].partial, int(blocks)};
+        return rc;
+    }
+
+    // Returns the buffer holding the level's final iterate and its pending
+    // mean (none: exact).  rhs_sum: the pending mean of the level's rhs.
+    int32_t level(int l, Pending rhs_sum, T** out, Pending* out_sum) {
+        int32_t rc;
+        *out_sum = none;
+        if (l >= first_cluster) return cluster(l, rhs_sum, out);
+        if (l >= first_coarse) return coarse(l, rhs_sum, out);
+        const Lv<T>& L = lv[l];
         T* cur = P(l);
         T* oth = Q(l);
+        Pending down_sum = none;
         for (int s = 0; s < plan->smooth; ++s) {
-            const bool first = s == 0;
-            const bool last = s == plan->smooth - 1;
-            if (zpairs(l))
-                rc = launch_pdl("mg sweep", sweep_zpair_kernel<BC, T>, gz.grid, gz.block, 0, stream,
-                                static_cast<const T*>((first && l > 0) ? nullptr : cur), R(l), oth, L,
-                                (first && l > 0 && singular) ? st.s[l][2].result : nullptr, st.s[l][0],
-                                (first && l > 0 && singular) ? 1 : 0, (last && singular) ? 1 : 0);
-            else
-                rc = launch_pdl("mg sweep", sweep_kernel<BC, false, T>, g.grid, g.block, 0, stream,
-                                (first && l > 0) ? nullptr : cur, R(l), oth, L, static_cast<const double*>(nullptr),
-                                (first && l > 0 && singular) ? st.s[l][2].result : nullptr, st.s[l][0],
-                                (first && l > 0 && singular) ? 1 : 0, (last && singular) ? 1 : 0);
+            const bool first = s == 0 && l > 0;
+            rc = sweep(l, first ? nullptr : cur, oth, first ? rhs_sum : none, 0, singular && s == plan->smooth - 1,
+                       &down_sum);
             if (rc) return rc;
             T* t = cur; cur = oth; oth = t;
         }
-        const double* down_sum = singular ? st.s[l][0].result : nullptr;
         const Lv<T>& C = lv[l + 1];
         const Geometry gc = launch_for(C, BC);
         if (zpairs(l))
             rc = launch_pdl("mg residual_restrict", residual_restrict_zpair_kernel<BC, T>, gc.grid, gc.block, 0, stream,
-                            cur, R(l), R(l + 1), L, C, down_sum, st.s[l + 1][2], singular ? 1 : 0);
+                            static_cast<const T*>(cur), static_cast<const T*>(R(l)), R(l + 1), L, C, down_sum,
+                            st.s[l + 1][2], singular ? 1 : 0);
         else
             rc = launch_pdl("mg residual_restrict", residual_restrict_kernel<BC, false, T>, gc.grid, gc.block, 0, stream,
-                            cur, R(l), R(l + 1), L, C, down_sum, st.s[l + 1][2], singular ? 1 : 0);
+                            static_cast<const T*>(cur), static_cast<const T*>(R(l)), R(l + 1), L, C, down_sum,
+                            st.s[l + 1][2], singular ? 1 : 0);
         if (rc) return rc;
         T* corr;
-        const double* corr_sum;
-        if ((rc = level(l + 1, &corr, &corr_sum))) return rc;
+        Pending corr_sum;
+        const Pending coarse_rhs = singular ? Pending{st.s[l + 1][2].partial, int(gc.blocks)} : none;
+        if ((rc = level(l + 1, coarse_rhs, &corr, &corr_sum))) return rc;
         // the finest level of a singular operator prolongs into the buffer the
         // pre-smoothing left free, so its post-smoothing ends in Q(0) and the
         // finalize (and the fused check of the solve loop) never shifts in place
         T* pdst = (l == 0 && singular && cur == P(l)) ? Q(l) : P(l);
-        rc = launch_pdl("mg prolong_add", prolong_kernel<BC, T>, g.grid, g.block, 0, stream, cur,
-                        static_cast<const T*>(corr), pdst, L, C, down_sum, corr_sum);
+        if (zpairs(l)) {
+            rc = launch_pdl("mg prolong_add", prolong_octet_kernel<BC, T>, gc.grid, gc.block, 0, stream,
+                            static_cast<const T*>(cur), static_cast<const T*>(corr), pdst, L, C, down_sum, corr_sum);
+        } else {
+            const Geometry g = launch_for(L, BC);
+            rc = launch_pdl("mg prolong_add", prolong_kernel<BC, T>, g.grid, g.block, 0, stream,
+                            static_cast<const T*>(cur), static_cast<const T*>(corr), pdst, L, C, down_sum, corr_sum);
+        }
         if (rc) return rc;
         cur = pdst;
         oth = pdst == P(l) ? Q(l) : P(l);
         for (int s = 0; s < plan->smooth; ++s) {
-            const bool last = s == plan->smooth - 1;
-            if (zpairs(l))
-                rc = launch_pdl("mg sweep", sweep_zpair_kernel<BC, T>, gz.grid, gz.block, 0, stream,
-                                static_cast<const T*>(cur), R(l), oth, L, static_cast<const double*>(nullptr),
-                                st.s[l][1], 0, (last && singular) ? 1 : 0);
-            else
-                rc = launch_pdl("mg sweep", sweep_kernel<BC, false, T>, g.grid, g.block, 0, stream, cur, R(l), oth,
-                                L, static_cast<const double*>(nullptr), static_cast<const double*>(nullptr),
-                                st.s[l][1], 0, (last && singular) ? 1 : 0);
-            if (rc) return rc;
+            if ((rc = sweep(l, cur, oth, none, 1, singular && s == plan->smooth - 1, out_sum))) return rc;
             T* t = cur; cur = oth; oth = t;
         }
         *out = cur;
-        *out_sum = singular ? st.s[l][1].result : nullptr;
         return AFSI_OK;
+    }
+
+    int32_t finalize(const T* out, Pending sum) {
+        return launch_pdl("mg finalize", shift_kernel<T>, dim3(flat_grid(lv[0].n)), dim3(kThreads), 0, stream, out, P(0),
+                          lv[0].n, sum);
     }
 
     int32_t cycles(int count) {
         for (int c = 0; c < count; ++c) {
             T* out;
-            const double* sum;
-            int32_t rc = level(0, &out, &sum);
+            Pending sum;
+            int32_t rc = level(0, none, &out, &sum);
             if (rc) return rc;
-            if (out != P(0) || sum) {
-                rc = launch_pdl("mg finalize", shift_kernel<T>, dim3(flat_grid(lv[0].n)), dim3(kThreads), 0, stream,
-                                static_cast<const T*>(out), P(0), lv[0].n, sum);
-                if (rc) return rc;
-            }
+            if ((out != P(0) || sum.part) && (rc = finalize(out, sum))) return rc;
         }
         return AFSI_OK;
     }
@@ -945,12 +1060,11 @@ struct Runner {
         int32_t rc = cycles(count - 1);
         if (rc) return rc;
         T* out;
-        const double* sum;
-        if ((rc = level(0, &out, &sum))) return rc;
+        Pending sum;
+        if ((rc = level(0, none, &out, &sum))) return rc;
         const Geometry g = launch_for(lv[0], BC);
-        if (out == P(0) && sum) {
-            rc = launch_pdl("mg finalize", shift_kernel<T>, dim3(flat_grid(lv[0].n)), dim3(kThreads), 0, stream,
-                            static_cast<const T*>(out), P(0), lv[0].n, sum);
+        if (out == P(0) && sum.part) {
+            rc = finalize(out, sum);
             if (!rc)
                 rc = launch_pdl("mg residual_norm", residual_norm_kernel<BC, true, T>, g.grid, g.block, 0, stream,
                                 static_cast<const T*>(P(0)), static_cast<const T*>(R(0)), lv[0], st.norm, norm);
@@ -1102,7 +1216,7 @@ struct RbRunner {
                                 static_cast<const T*>(x), lv[l], site);
         if (rc) return rc;
         return launch_pdl("mg mean shift", shift_kernel<T>, dim3(flat_grid(lv[l].n)), dim3(kThreads), 0, stream,
-                          static_cast<const T*>(x), x, lv[l].n, static_cast<const double*>(site.result));
+                          static_cast<const T*>(x), x, lv[l].n, Pending{site.result, 1});
     }
 
     int32_t level(int l) {
@@ -1117,12 +1231,12 @@ struct RbRunner {
         const Geometry gc = launch_for(lv[l + 1], BC);
         rc = launch_pdl("mg residual restrict", residual_restrict_kernel<BC, true, T>, gc.grid, gc.block, 0, stream,
                         static_cast<const T*>(P(l)), static_cast<const T*>(R(l)), R(l + 1), lv[l], lv[l + 1],
-                        static_cast<const double*>(nullptr), st.s[l + 1][2], int(singular));
+                        Pending{nullptr, 0}, st.s[l + 1][2], int(singular));
         if (rc) return rc;
         if (singular) {
             rc = launch_pdl("mg mean shift", shift_kernel<T>, dim3(flat_grid(lv[l + 1].n)), dim3(kThreads), 0, stream,
                             static_cast<const T*>(R(l + 1)), R(l + 1), lv[l + 1].n,
-                            static_cast<const double*>(st.s[l + 1][2].result));
+                            Pending{st.s[l + 1][2].partial, int(gc.blocks)});
             if (rc) return rc;
         }
         if (l + 1 < last && l + 1 != first_coarse) {
@@ -1133,7 +1247,7 @@ struct RbRunner {
         const Geometry g = launch_for(lv[l], BC);
         rc = launch_pdl("mg prolong add", prolong_kernel<BC, T>, g.grid, g.block, 0, stream,
                         static_cast<const T*>(P(l)), static_cast<const T*>(P(l + 1)), P(l), lv[l], lv[l + 1],
-                        static_cast<const double*>(nullptr), static_cast<const double*>(nullptr));
+                        Pending{nullptr, 0}, Pending{nullptr, 0});
         if (rc) return rc;
         return smooth(l);
     }
@@ -1444,7 +1558,7 @@ extern "C" int32_t afsi_b200_subtract_mean(void* x, int64_t n, const double* sta
     AFSI_REQUIRE(n > 0 && x && stats, "invalid subtract_mean arguments");
     AFSI_DISPATCH(dtype, {
         shift_kernel<T><<<flat_grid(n), kThreads, 0, stream>>>(static_cast<const T*>(x), static_cast<T*>(x), n,
-                                                               stats);
+                                                               Pending{stats, 1});
     });
     return launched("subtract_mean");
 }
@@ -1499,7 +1613,7 @@ extern "C" int32_t afsi_b200_mg_smooth(const void* p, const void* rhs, void* out
             Site none{nullptr, nullptr, nullptr};
             sweep_kernel<BC, true, T><<<g.grid, g.block, 0, stream>>>(
                 static_cast<const T*>(p), const_cast<T*>(static_cast<const T*>(rhs)), static_cast<T*>(out), L,
-                nullptr, nullptr, none, 0, 0);
+                Pending{nullptr, 0}, Pending{nullptr, 0}, none, 0, 0);
         });
     });
     return launched("mg_smooth");
@@ -1560,8 +1674,8 @@ extern "C" int32_t afsi_b200_mg_residual_restrict(const void* p, const void* rhs
             const Geometry g = launch_for(C, BC);
             Site none{nullptr, nullptr, nullptr};
             residual_restrict_kernel<BC, true, T><<<g.grid, g.block, 0, stream>>>(
-                static_cast<const T*>(p), static_cast<const T*>(rhs), static_cast<T*>(coarse), L, C, nullptr, none,
-                0);
+                static_cast<const T*>(p), static_cast<const T*>(rhs), static_cast<T*>(coarse), L, C, Pending{nullptr, 0},
+                none, 0);
         });
     });
     return launched("mg_residual_restrict");
@@ -1581,7 +1695,7 @@ extern "C" int32_t afsi_b200_mg_prolong_add(const void* coarse, void* fine, cons
             const Geometry g = launch_for(L, BC);
             prolong_kernel<BC, T><<<g.grid, g.block, 0, stream>>>(static_cast<const T*>(fine),
                                                                   static_cast<const T*>(coarse), static_cast<T*>(fine),
-                                                                  L, C, nullptr, nullptr);
+                                                                  L, C, Pending{nullptr, 0}, Pending{nullptr, 0});
         });
     });
     return launched("mg_prolong_add");
@@ -1920,7 +2034,7 @@ __global__ void __launch_bounds__(kCoarseThreads) batch_coarse_kernel(const Batc
     const TC* cinv = j.cinv;
     __syncthreads();
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    coarse_cycle<BC, T, TC>(reinterpret_cast<T*>(smem_raw), rhs, nullptr, p_start, p_out, cinv, cl, smooth);
+    coarse_cycle<BC, T, TC>(reinterpret_cast<T*>(smem_raw), rhs, Pending{nullptr, 0}, p_start, p_out, cinv, cl, smooth);
 }
 
 // ---- persistent batched V-cycles: every level operation of every cycle in
@@ -1986,7 +2100,7 @@ __global__ void __launch_bounds__(kBatchPThreads, 1) batch_persistent_kernel(Bat
             unsigned* dst = reinterpret_cast<unsigned*>(&cl);
             for (int k = threadIdx.x; k < int(sizeof(cl) / 4); k += blockDim.x) dst[k] = src[k];
             __syncthreads();
-            coarse_cycle<BC, T, TC>(reinterpret_cast<T*>(smem_raw), jobs[j].rhs, nullptr, jobs[j].p_start,
+            coarse_cycle<BC, T, TC>(reinterpret_cast<T*>(smem_raw), jobs[j].rhs, Pending{nullptr, 0}, jobs[j].p_start,
                                     jobs[j].p_out, jobs[j].cinv, cl, a.smooth);
             __syncthreads();
         }

@@ -166,11 +166,11 @@ __device__ void cluster_tables(T* arena, const ClusterLevels<T>& cl) {
 }
 
 // Levels first..last of one V-cycle in a cluster (3D BCs).  As coarse_cycle:
-// rhs of level `first` from global memory (shifted by rhs_sum/n), p from
+// rhs of level `first` from global memory (shifted by its pending mean), p from
 // p_global (first == 0) or zero; the final p of level `first`, mean removed
 // for the singular operator, written to p_out.  Level `first` is distributed.
 template <int BC, class T, class TC>
-__device__ void cluster_cycle(T* arena, const T* __restrict__ rhs_global, const double* rhs_sum, const T* p_global,
+__device__ void cluster_cycle(T* arena, const T* __restrict__ rhs_global, Pending rhs_sum, const T* p_global,
                               T* p_out, const TC* __restrict__ cinv, const ClusterLevels<T>& cl, int smooth) {
     __shared__ double red[2][32];
     __shared__ double slot[2], bcast[2];
@@ -184,7 +184,7 @@ __device__ void cluster_cycle(T* arena, const T* __restrict__ rhs_global, const 
     T* tables = arena + cl.tables;  // filled by cluster_tables before the kernel waits on its predecessor
     {
         const ClusterLevel<T>& lv = cl.lv[f];
-        const T mr = T(site_mean(rhs_sum, lv.L.n));
+        const T mr = T(pending_mean(rhs_sum, lv.L.n));
         T* P = P_of(f);
         T* R = P + 2 * lv.cells;
         const int64_t g0 = int64_t(rank) * lv.cells;

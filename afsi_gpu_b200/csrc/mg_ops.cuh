@@ -249,10 +249,6 @@ __device__ __forceinline__ void coords32(int i, const Lv<T>& L, int& x, int& y, 
 template <class T>
 __host__ __device__ __forceinline__ T omega() { return T(2.0 / 3.0); }
 
-__device__ __forceinline__ double site_mean(const double* result, int64_t n) {
-    return result ? *result / double(n) : 0.0;
-}
-
 __device__ __forceinline__ unsigned block_linear() {
     return blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
 }
@@ -271,6 +267,44 @@ __device__ __forceinline__ double block_sum2(double v, double* shared) {
     if (warp == 0) v = warp_sum(v);
     __syncthreads();
     return v;
+}
+
+// A pending mean: the sum, over `count` doubles, of a field that its producer
+// left as one partial per block (or, count 1, a finished sum); part == nullptr:
+// none.
+struct Pending {
+    const double* part;
+    int count;
+};
+
+// Mean of a pending sum over n cells, the same bits in every thread of every
+// block whatever the block's size: warp 0 adds partials l, l + 32, ... per lane
+// and then a fixed tree.  Summing a few hundred partials in each consumer
+// block costs one L2 round trip; completing the sum in the producer cost a
+// fence, a counter and a last block at the end of every emitting launch.
+__device__ __forceinline__ double pending_mean(Pending s, int64_t n) {
+    if (!s.part) return 0.0;
+    __shared__ double mean;
+    const unsigned t = thread_linear();
+    if (t < 32) {
+        double v = 0.0;
+#pragma unroll 4
+        for (int i = int(t); i < s.count; i += 32) v += __ldcg(s.part + i);
+#pragma unroll
+        for (int d = 16; d; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
+        if (t == 0) mean = v / double(n);
+    }
+    __syncthreads();
+    const double m = mean;
+    __syncthreads();  // `mean` is reused by the next call
+    return m;
+}
+
+// This block's share of a field's sum, left for pending_mean.
+__device__ __forceinline__ void site_put(const Site& s, double v) {
+    __shared__ double warp_sums[32];
+    v = block_sum2(v, warp_sums);
+    if (thread_linear() == 0) s.partial[block_linear()] = v;
 }
 
 // Block partial + last-block completion for a grid reduction of `v`.
@@ -600,12 +634,12 @@ __device__ T* block_smooth(T* cur, T* oth, T* R, const Lv<T>& L, const FastCoord
 }
 
 // Levels first..last of one V-cycle in one CTA (fast arithmetic).  rhs of
-// level `first` comes from global memory (shifted by rhs_sum/n); p[first]
+// level `first` comes from global memory (shifted by its pending mean); p[first]
 // starts from p_global (first==0) or zero; the final p[first], mean removed
 // for the singular operators, is written to p_out.  smem holds, per level, p,
 // its Jacobi partner and rhs, then the omega/diag tables.
 template <int BC, class T, class TC>
-__device__ void coarse_cycle(T* smem, const T* __restrict__ rhs_global, const double* rhs_sum, const T* p_global,
+__device__ void coarse_cycle(T* smem, const T* __restrict__ rhs_global, Pending rhs_sum, const T* p_global,
                              T* p_out, const TC* __restrict__ cinv, const CoarseLevels<T>& cl, int smooth) {
     __shared__ double red[2][32];
     __shared__ T down_mean[AFSI_MG_MAX_LEVELS];  // pending mean of each level's pre-smoothed iterate
@@ -621,7 +655,7 @@ __device__ void coarse_cycle(T* smem, const T* __restrict__ rhs_global, const do
     T* tables = level_base(last + 1);
     for (int l = f; l <= last; ++l) omega_table<BC>(cl.lv[l], tables + 64 * (l - f));
     {
-        const T mr = T(site_mean(rhs_sum, cl.lv[f].n));
+        const T mr = T(pending_mean(rhs_sum, cl.lv[f].n));
         T* P = level_base(f);
         T* R = P + 2 * cl.lv[f].n;
         for (int i = threadIdx.x; i < cl.lv[f].n; i += blockDim.x) {

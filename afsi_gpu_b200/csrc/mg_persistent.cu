@@ -150,7 +150,8 @@ __global__ void __launch_bounds__(kPThreads, 1) mg_persistent(PersistentArgs<T, 
         // ---- coarse levels in block 0
         if (blockIdx.x == 0)
             coarse_cycle<BC, T, TC>(reinterpret_cast<T*>(smem_raw), a.R[fc],
-                                    (fc > 0 && singular) ? gs.slot + fc * 3 + 2 : nullptr, fc == 0 ? a.P[0] : nullptr,
+                                    Pending{(fc > 0 && singular) ? gs.slot + fc * 3 + 2 : nullptr, 1},
+                                    fc == 0 ? a.P[0] : nullptr,
                                     a.P[fc], a.cinv, a.coarse, a.smooth);
         ok = grid_sync(gs, 0.0, nullptr);
         const T* corr = a.P[fc];
