@@ -123,15 +123,26 @@ __device__ T* dist_smooth(T* cur, T* oth, T* R, const ClusterLevel<T>& lv, const
     constexpr bool singular = singular_bc(BC);
     const Lv<T>& L = lv.L;
     const int x0 = rank * lv.ppc;
+    // the thread's first cell (its only one up to 1024 cells per CTA): coordinates
+    // (three divisions) and weight found once and not in every sweep
+    int fx = 0, fy = 0, fz = 0;
+    T fw = T(0);
+    if (int(threadIdx.x) < lv.cells) {
+        slab_coords(int(threadIdx.x), L, fx, fy, fz);
+        fw = wrd[boundary_class(x0 + fx, fy, fz, L.nx, L.ny, L.nz)];
+    }
     for (int s = 0; s < smooth; ++s) {
         const bool last = s == smooth - 1;
         const bool z0 = s == 0 && zero;
         const Slab<T> h = slab_of<T>(cur, rank, ranks);
         double acc = 0.0;
         for (int i = threadIdx.x; i < lv.cells; i += blockDim.x) {
-            int xl, y, z;
-            slab_coords(i, L, xl, y, z);
-            const T w = wrd[boundary_class(x0 + xl, y, z, L.nx, L.ny, L.nz)];
+            int xl = fx, y = fy, z = fz;
+            T w = fw;
+            if (i != int(threadIdx.x)) {
+                slab_coords(i, L, xl, y, z);
+                w = wrd[boundary_class(x0 + xl, y, z, L.nx, L.ny, L.nz)];
+            }
             T v;
             if (z0) {
                 const T r = R[i] - rhs_shift;
