@@ -25,15 +25,21 @@
 // Layout: one warp per element, the three components in turn.  The element's
 // point positions are formed once (lanes over points, kept in shared memory
 // for rules of at most one chunk); per component, lanes over points form the
-// three weight rows the component reads (x, y, z: 12 values per point), its
-// support origins and, for the spread, its force factors; the warp reduces
-// the component's box.  The spread then accumulates runs of points with one
-// support origin in registers and adds each run to a padded shared-memory box
-// once (spread_runs, runs.cuh), flushed to the face array with one L2
+// three weight rows the component reads (x, y, z: 12 values per point) and its
+// support origins; the warp reduces the component's box.  The spread groups the
+// points by support origin and adds each group to a padded shared-memory box
+// once (spread_element, runs.cuh), flushed to the face array with one L2
 // reduction per non-zero face.  The gather stages the component's face patch
-// in the same padded layout, and four lane groups of eight walk contiguous
-// quarters of the points, reloading their eight patch values only when the
-// support origin changes.  A point whose support leaves the grid sets
+// and sums one point per lane over it.
+//
+// Bound by instruction issue and dependent latency at 16 warps per SM (56 % and
+// 49 % active).  38,400 P2 elements of 64 points on 64^3, FP64, one B200: spread
+// 433 -> 403 us and gather 295 -> 280 us with each basis row read once and by
+// pairs (the rows of a warp's points touch a sector per lane: 101 M sectors and an
+// L1 71 % busy before), the force factors of the three components formed
+// together, 7 rows per point instead of 9 in the spread, the groups placed by a
+// scan and the boxes reduced by redux.  Keeping the row that two components share
+// in shared memory made the gather slower (287 us).  A point whose support leaves the grid sets
 // AFSI_FLAG_SUPPORT and is skipped; an element with a node id outside
 // [0, nodes) sets AFSI_FLAG_INDEX and is skipped.
 #include <algorithm>
@@ -70,10 +76,6 @@ struct FBox {
     int lo[3], ext[3];
 };
 
-template <class T> struct FPair;
-template <> struct FPair<double> { using type = double2; };
-template <> struct FPair<float> { using type = float2; };
-
 // (x - start) / h on lattice l of axis a.
 template <class TP>
 __device__ __forceinline__ TP lattice_scaled(const Geo<TP>& geo, TP x, int a, int l) {
@@ -86,13 +88,13 @@ __device__ __forceinline__ TP lattice_scaled(const Geo<TP>& geo, TP x, int a, in
 template <class TP, int NPC>
 __device__ __forceinline__ bool point_position(const TP* __restrict__ Npos, const TP* xs, int64_t q,
                                                const Geo<TP>& geo, TP pos[3]) {
+    TP row[NPC];
+    basis_row<TP, NPC>(Npos, q, row);
     pos[0] = pos[1] = pos[2] = TP(0);
 #pragma unroll
-    for (int a = 0; a < NPC; ++a) {
-        const TP nv = Npos[q * NPC + a];
+    for (int a = 0; a < NPC; ++a)
 #pragma unroll
-        for (int d = 0; d < 3; ++d) pos[d] += nv * xs[a * 3 + d];
-    }
+        for (int d = 0; d < 3; ++d) pos[d] += row[a] * xs[a * 3 + d];
     bool valid = true;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
@@ -102,22 +104,18 @@ __device__ __forceinline__ bool point_position(const TP* __restrict__ Npos, cons
     return valid;
 }
 
-// Component c's support origins of a point (axis a on lattice a != c) and,
-// with w != null, its weight rows w[a*4 + k].
-template <class TP, class T>
-__device__ __forceinline__ void component_rows(const Geo<TP>& geo, const TP pos[3], int c, int b[3], T* w) {
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        const TP scaled = lattice_scaled(geo, pos[a], a, a != c);
-        const int64_t lower = static_cast<int64_t>(floor(scaled - TP(1)));
-        b[a] = int(lower);
-        if (w) {
-            TP r[4];
-            peskin_radical(scaled - TP(lower) - TP(1), r);
-#pragma unroll
-            for (int k = 0; k < 4; ++k) w[a * 4 + k] = T(r[k]);
-        }
-    }
+template <class TP>
+__device__ __forceinline__ int axis_origin(TP scaled) {
+    return int(static_cast<int64_t>(floor(scaled - TP(1))));
+}
+
+// Row of axis a on lattice l: support origin and, in r, the four weights.
+template <class TP>
+__device__ __forceinline__ int axis_row(const Geo<TP>& geo, TP pos, int a, int l, TP r[4]) {
+    const TP scaled = lattice_scaled(geo, pos, a, l);
+    const int64_t lower = static_cast<int64_t>(floor(scaled - TP(1)));
+    peskin_radical(scaled - TP(lower) - TP(1), r);
+    return int(lower);
 }
 
 __device__ __forceinline__ void bounds_init(int mn[3], int mx[3]) {
@@ -139,14 +137,9 @@ __device__ __forceinline__ void bounds_add(int mn[3], int mx[3], const int b[3])
 // Warp-reduce the per-lane bounds into the box; false when no point was valid.
 __device__ __forceinline__ bool bounds_finish(int mn[3], int mx[3], FBox& bx) {
 #pragma unroll
-    for (int a = 0; a < 3; ++a)
-#pragma unroll
-        for (int d = 16; d; d >>= 1) {
-            mn[a] = min(mn[a], __shfl_xor_sync(0xffffffffu, mn[a], d));
-            mx[a] = max(mx[a], __shfl_xor_sync(0xffffffffu, mx[a], d));
-        }
-#pragma unroll
     for (int a = 0; a < 3; ++a) {
+        mn[a] = __reduce_min_sync(0xffffffffu, mn[a]);
+        mx[a] = __reduce_max_sync(0xffffffffu, mx[a]);
         bx.lo[a] = mn[a];
         bx.ext[a] = mx[a] == INT_MIN ? 0 : mx[a] - mn[a] + 4;
     }
@@ -223,12 +216,13 @@ struct __align__(16) FStage {
     TP pos[FChunk<NPC>::value * 3];    // positions of a resident rule
     int b[FChunk<NPC>::value * 3];     // support origins (absolute) of the component
     int key[FChunk<NPC>::value];       // run keys in the box, -1 for an invalid point
-    T f[FChunk<NPC>::value + 1];       // spread: force factors of the component; the last stays zero
+    T f[3][FChunk<NPC>::value + 1];    // force factors per component; the last stays zero
     T box[Cap];                        // padded box
     T coef[32];
     TP xs[32];
-    int perm[4 * FChunk<NPC>::value];  // points grouped by key (spread_element)
-    int rs[FChunk<NPC>::value + 1], rk[FChunk<NPC>::value];
+    int rk[FChunk<NPC>::value];             // points grouped by key (spread_element)
+    uint16_t rs[FChunk<NPC>::value + 1];
+    uint8_t perm[4 * FChunk<NPC>::value];
 };
 
 // Positions of a resident rule (all nq <= chunk points) into s.pos; returns
@@ -271,7 +265,8 @@ __device__ __forceinline__ bool component_box_all(const TP* __restrict__ Npos, c
             continue;
         }
         int b[3];
-        component_rows<TP, float>(geo, pos, c, b, nullptr);
+#pragma unroll
+        for (int a = 0; a < 3; ++a) b[a] = axis_origin(lattice_scaled(geo, pos[a], a, a != c));
         bounds_add(mn, mx, b);
     }
     if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) flag(status, AFSI_FLAG_SUPPORT);
@@ -279,16 +274,20 @@ __device__ __forceinline__ bool component_box_all(const TP* __restrict__ Npos, c
 }
 
 // Rows pass of component c over points q0 .. q0+n-1 (lanes over points):
-// weight rows and absolute support origins into shared memory, the spread's
-// force factors when coef != null; the bounds of the valid points' origins
-// are added to mn/mx.  Invalid points get b[q*3] = INT_MIN.
+// weight rows and absolute support origins into shared memory; the bounds of
+// the valid points' origins are added to mn/mx.  Invalid points get
+// b[q*3] = INT_MIN.  A resident rule (one chunk) keeps what the components
+// share: the first one visited forms the force factors of all three from one
+// reading of the point's basis row, and the row of the axis that keeps its
+// lattice (z from component 0 to 1, x from 1 to 2) stays.
 template <class TP, class T, int NPC, int Cap>
 __device__ __forceinline__ void component_pass(FStage<TP, T, NPC, Cap>& s, const TP* __restrict__ Npos,
                                                const T* __restrict__ N, const T* __restrict__ W, bool resident,
                                                unsigned long long valid_bits, int64_t e, int64_t nq, int64_t q0,
-                                               int n, const Geo<TP>& geo, int c, const T* coef, T volume, T inv_volume, int mn[3],
-                                               int mx[3]) {
+                                               int n, const Geo<TP>& geo, int c, bool first, T volume, T inv_volume,
+                                               int mn[3], int mx[3]) {
     const int lane = threadIdx.x & 31;
+    const int keep = resident && !first ? (c == 1 ? 2 : 0) : -1;
 #pragma unroll 1
     for (int j = 0; j < FChunk<NPC>::value / 32; ++j) {
         const int q = lane + 32 * j;
@@ -307,16 +306,32 @@ __device__ __forceinline__ void component_pass(FStage<TP, T, NPC, Cap>& s, const
             continue;
         }
         int b[3];
-        component_rows<TP, T>(geo, pos, c, b, &s.w[q * 12]);
 #pragma unroll
-        for (int a = 0; a < 3; ++a) s.b[q * 3 + a] = b[a];
+        for (int a = 0; a < 3; ++a) {
+            if (a == keep) {
+                b[a] = s.b[q * 3 + a];
+            } else {
+                TP r[4];
+                b[a] = axis_row(geo, pos[a], a, a != c, r);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) s.w[q * 12 + a * 4 + k] = T(r[k]);
+                s.b[q * 3 + a] = b[a];
+            }
+        }
         bounds_add(mn, mx, b);
-        if (coef) {
-            T F = T(0);
+        if (first || !resident) {
+            T row[NPC];
+            basis_row<T, NPC>(N, q0 + q, row);
+            const T wq = W[e * nq + q0 + q];
 #pragma unroll
-            for (int a = 0; a < NPC; ++a) F += N[(q0 + q) * NPC + a] * coef[a * 3 + c];
-            const T fw = F * W[e * nq + q0 + q];
-            s.f[q] = inv_volume != T(0) ? fw * inv_volume : fw / volume;
+            for (int d = 0; d < 3; ++d) {
+                if (!resident && d != c) continue;
+                T F = T(0);
+#pragma unroll
+                for (int a = 0; a < NPC; ++a) F += row[a] * s.coef[a * 3 + d];
+                const T fw = F * wq;
+                s.f[d][q] = inv_volume != T(0) ? fw * inv_volume : fw / volume;
+            }
         }
     }
 }
@@ -365,7 +380,7 @@ __global__ void __launch_bounds__(kFWarps * 32, 8) fused_spread_kernel(
     const bool resident = g.nq <= C;
     const T inv_volume = exact_reciprocal(volume);
     if (lane < 12) s.w[C * 12 + lane] = T(0);
-    if (lane == 0) s.f[C] = T(0);
+    if (lane < 3) s.f[lane][C] = T(0);
     __syncwarp();
     const int64_t items = Mode == 2 ? int64_t(*queued) : g.elements;
     for (int64_t it = int64_t(blockIdx.x) * kFWarps + (threadIdx.x >> 5); it < items; it += warps) {
@@ -389,8 +404,8 @@ __global__ void __launch_bounds__(kFWarps * 32, 8) fused_spread_kernel(
                 __syncwarp();
                 int mn[3], mx[3];
                 bounds_init(mn, mx);
-                component_pass(s, Npos, N, W, resident, valid, e, g.nq, q0, n, geo, c, s.coef, volume,
-                                           inv_volume, mn, mx);
+                component_pass(s, Npos, N, W, resident, valid, e, g.nq, q0, n, geo, c, c == 0 || Mode == 2, volume,
+                               inv_volume, mn, mx);
                 if (resident) {
                     any = bounds_finish(mn, mx, bx);
                     if (!any) break;
@@ -405,7 +420,7 @@ __global__ void __launch_bounds__(kFWarps * 32, 8) fused_spread_kernel(
                 component_keys(s, n, bx, fits);
                 __syncwarp();
                 if (fits) {
-                    spread_element<T, C>(s.box, s.key, s.f, s.w, s.w + 4, s.w + 8, n, sx, sy, s.perm, s.rs, s.rk);
+                    spread_element<T, C>(s.box, s.key, s.f[c], s.w, s.w + 4, s.w + 8, n, sx, sy, s.perm, s.rs, s.rk);
                 } else if (Mode == 1) {
                     if (lane == 0) queue[atomicAdd(queued, 1)] = int32_t(e * 3 + c);
                     break;
@@ -417,7 +432,7 @@ __global__ void __launch_bounds__(kFWarps * 32, 8) fused_spread_kernel(
                         const int gx = s.b[q * 3], gy = s.b[q * 3 + 1], gz = s.b[q * 3 + 2];
                         if (gx == INT_MIN) continue;
                         if (fpoint_inside(g, c, gx, gy, gz)) {
-                            const T w = (s.w[q * 12 + li] * s.w[q * 12 + 4 + lj]) * s.f[q];
+                            const T w = (s.w[q * 12 + li] * s.w[q * 12 + 4 + lj]) * s.f[c][q];
                             T* dst = field + ffield_index(g, c, gx + li, gy + lj, gz);
 #pragma unroll
                             for (int k = 0; k < 4; ++k) atomicAdd(dst + k, w * s.w[q * 12 + 8 + k]);
@@ -862,15 +877,6 @@ __device__ __forceinline__ unsigned stage_elements(const TP* __restrict__ x, con
     return ok;
 }
 
-// Row of axis a on lattice l: support origin and, in r, the four weights.
-template <class TP>
-__device__ __forceinline__ int axis_row(const Geo<TP>& geo, TP pos, int a, int l, TP r[4]) {
-    const TP scaled = lattice_scaled(geo, pos, a, l);
-    const int64_t lower = static_cast<int64_t>(floor(scaled - TP(1)));
-    peskin_radical(scaled - TP(lower) - TP(1), r);
-    return int(lower);
-}
-
 template <class T>
 __device__ __forceinline__ void store_row(T* dst, const T w[4]) {  // dst 16-byte aligned
     if constexpr (sizeof(T) == 8) {
@@ -969,13 +975,12 @@ __global__ void __launch_bounds__(kMWarps * 32, 4) fused_spread_multi_kernel(
                 if ((ok >> el[j]) & 1u) {
                     live[j] = point_position<TP, NPC>(Npos, s.xs + el[j] * NPC * 3, q, geo, pos[j]);
                     if (!live[j]) flag(status, AFSI_FLAG_SUPPORT);
-                    T F[3] = {T(0), T(0), T(0)};
+                    T F[3] = {T(0), T(0), T(0)}, nrow[NPC];
+                    basis_row<T, NPC>(N, q, nrow);
 #pragma unroll
-                    for (int a = 0; a < NPC; ++a) {
-                        const T nv = N[q * NPC + a];
+                    for (int a = 0; a < NPC; ++a)
 #pragma unroll
-                        for (int c = 0; c < 3; ++c) F[c] += nv * s.coef[(el[j] * NPC + a) * 3 + c];
-                    }
+                        for (int c = 0; c < 3; ++c) F[c] += nrow[a] * s.coef[(el[j] * NPC + a) * 3 + c];
                     const T wq = W[e0 * nq + p];
 #pragma unroll
                     for (int c = 0; c < 3; ++c) {

@@ -633,7 +633,7 @@ __device__ T* block_smooth(T* cur, T* oth, T* R, const Lv<T>& L, const FastCoord
     // kCoarseCells and 1024 threads), found once and not in every sweep: a
     // sweep is bound by this SM's issue rate, and the coordinates of a cell (two
     // divisions where extents are not powers of two) cost as much as its update
-    // (12 cycles' solve on 256 x 64, one B200: 732 -> 705 us; on 64^3 1190 -> 1163)
+    // (a solve of 12 cycles on 256 x 64, one B200: 732 -> 705 us)
     const auto class_of = [&](int i) {
         int x, y, z;
         fc.get(i, L, x, y, z);

@@ -22,8 +22,12 @@
 // per element for the deterministic node reduction).
 // Rules of at most 64 points per element take a spread variant that stages the
 // element's stencil rows in shared memory with bulk copies first and merges
-// runs of points with the same support origin in registers before adding them
-// to a single box copy (p2_spread_rows_kernel, runs.cuh).
+// the points with the same support origin before adding them to a single box
+// copy (p2_spread_rows_kernel, runs.cuh).  12 warps per SM bound it (20 KB of
+// shared memory each); 38,400 elements of 64 points, FP64, one B200: 488 -> 479 us
+// with the basis rows read once, the groups placed by a scan and the boxes reduced
+// by redux (the gather 311 -> 301).  Rows kept from one component to the next made
+// the gather slower (342 us: bound by the shared-memory pipe).
 // Point forces F = (Σ_a N[q,a] value[a]) * W (mac/compact_transfer.py:29-35)
 // are computed once per point and component by a lanes-over-points pass; the
 // spread contribution is (φx·φy)·φz · (F/volume), one division per point
@@ -104,11 +108,8 @@ __device__ __forceinline__ void element_box(const int64_t* __restrict__ base, co
     for (int c = 0; c < 3; ++c)
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
-#pragma unroll
-            for (int d = 16; d; d >>= 1) {
-                mn[c][a] = min(mn[c][a], __shfl_xor_sync(0xffffffffu, mn[c][a], d));
-                mx[c][a] = max(mx[c][a], __shfl_xor_sync(0xffffffffu, mx[c][a], d));
-            }
+            mn[c][a] = __reduce_min_sync(0xffffffffu, mn[c][a]);
+            mx[c][a] = __reduce_max_sync(0xffffffffu, mx[c][a]);
             bx.lo[c][a] = mn[c][a];
             bx.ext[c][a] = mx[c][a] - mn[c][a] + 4;
         }
@@ -316,12 +317,12 @@ template <class T>
 struct __align__(16) RowStage {  // size a multiple of 16: every warp's copy targets start 16-byte aligned
     T phi[2][(kRowPoints + 1) * 12];  // row kRowPoints stays zero (spread_element's padding row)
     int64_t base[2][kRowPoints * 3];
-    T f[kRowPoints + 1];
+    T f[3][kRowPoints + 1];
     T coef[32];
     T box[kSpreadCap];
-    int key[kRowPoints];
-    int perm[4 * kRowPoints];   // points grouped by key (spread_element)
-    int rs[kRowPoints + 1], rk[kRowPoints];
+    int key[kRowPoints], rk[kRowPoints];  // points grouped by key (spread_element)
+    uint16_t rs[kRowPoints + 1];
+    uint8_t perm[4 * kRowPoints];
     unsigned long long bar;  // completion of this warp's bulk copies
 };
 
@@ -341,7 +342,7 @@ __global__ void __launch_bounds__(kRowWarps * 32, 6) p2_spread_rows_kernel(
     const bool phi_bulk = phi_bytes % 16 == 0;
     if (lane == 0) mbar_init(&s.bar);
     if (lane < 24) s.phi[lane / 12][kRowPoints * 12 + lane % 12] = T(0);
-    if (lane == 0) s.f[kRowPoints] = T(0);
+    if (lane < 3) s.f[lane][kRowPoints] = T(0);
     __syncwarp();
     unsigned parity = 0;
     for (int64_t e = int64_t(blockIdx.x) * kRowWarps + (threadIdx.x >> 5); e < g.elements; e += warps) {
@@ -416,11 +417,8 @@ __global__ void __launch_bounds__(kRowWarps * 32, 6) p2_spread_rows_kernel(
             for (int c = 0; c < 3; ++c)
 #pragma unroll
                 for (int a = 0; a < 3; ++a) {
-#pragma unroll
-                    for (int d = 16; d; d >>= 1) {
-                        mn[c][a] = min(mn[c][a], __shfl_xor_sync(0xffffffffu, mn[c][a], d));
-                        mx[c][a] = max(mx[c][a], __shfl_xor_sync(0xffffffffu, mx[c][a], d));
-                    }
+                    mn[c][a] = __reduce_min_sync(0xffffffffu, mn[c][a]);
+                    mx[c][a] = __reduce_max_sync(0xffffffffu, mx[c][a]);
                     bx.lo[c][a] = mn[c][a];
                     bx.ext[c][a] = mx[c][a] - mn[c][a] + 4;
                 }
@@ -434,19 +432,28 @@ __global__ void __launch_bounds__(kRowWarps * 32, 6) p2_spread_rows_kernel(
             __syncwarp();
             if (fits)
                 for (int t = lane; t < kSpreadCap; t += 32) s.box[t] = T(0);
-            for (int q = lane; q < n; q += 32) {  // component c of the forces and the run keys, lanes over points
-                T F = T(0);
+            for (int q = lane; q < n; q += 32) {  // the forces (once) and the run keys, lanes over points
+                if (c == 0) {
+                    T row[10];
+                    basis_row<T, 10>(N, q, row);
+                    const T wq = W[e * g.nq + q];
 #pragma unroll
-                for (int a = 0; a < 10; ++a) F += N[q * 10 + a] * s.coef[a * 3 + c];
-                const T fw = F * W[e * g.nq + q];
-                s.f[q] = inv_volume != T(0) ? fw * inv_volume : fw / volume;
+                    for (int d = 0; d < 3; ++d) {
+                        T F = T(0);
+#pragma unroll
+                        for (int a = 0; a < 10; ++a) F += row[a] * s.coef[a * 3 + d];
+                        const T fw = F * wq;
+                        s.f[d][q] = inv_volume != T(0) ? fw * inv_volume : fw / volume;
+                    }
+                }
                 if (fits)
                     s.key[q] = run_key(int(s.base[tx][q * 3]) - bx.lo[c][0], int(s.base[ty][q * 3 + 1]) - bx.lo[c][1],
                                        int(s.base[tz][q * 3 + 2]) - bx.lo[c][2]);
             }
             __syncwarp();
             if (fits) {
-                spread_element<T, kRowPoints>(s.box, s.key, s.f, s.phi[tx], s.phi[ty] + 4, s.phi[tz] + 8, n, sx, sy, s.perm, s.rs, s.rk);
+                spread_element<T, kRowPoints>(s.box, s.key, s.f[c], s.phi[tx], s.phi[ty] + 4, s.phi[tz] + 8, n, sx, sy,
+                                              s.perm, s.rs, s.rk);
                 __syncwarp();
                 box_walk(lane, bx.ext[c][0], bx.ext[c][1], bx.ext[c][2], [&](int, int x, int y, int z) {
                     const T v = s.box[x * sx + y * sy + z];
@@ -458,7 +465,7 @@ __global__ void __launch_bounds__(kRowWarps * 32, 6) p2_spread_rows_kernel(
                     const int gx = int(s.base[tx][q * 3]), gy = int(s.base[ty][q * 3 + 1]),
                               gz = int(s.base[tz][q * 3 + 2]);
                     if (point_inside(g, c, gx, gy, gz)) {
-                        const T w = (s.phi[tx][q * 12 + li] * s.phi[ty][q * 12 + 4 + lj]) * s.f[q];
+                        const T w = (s.phi[tx][q * 12 + li] * s.phi[ty][q * 12 + 4 + lj]) * s.f[c][q];
                         T* dst = field + face_index(g, c, gx + li, gy + lj, gz);
 #pragma unroll
                         for (int k = 0; k < 4; ++k) atomicAdd(dst + k, w * s.phi[tz][q * 12 + 8 + k]);

@@ -83,9 +83,12 @@ __device__ __forceinline__ void spread_runs(T* box, const int* key, const T* f, 
 // among points j*32 .. j*32+31 in index order, padded with `zero` (the index of
 // an all-zero row) to a multiple of four; run r spans perm[rs[r] .. rs[r+1])
 // and has key rk[r].  Points with key < 0 take no part.  perm needs room for
-// 4 n entries.  Returns the number of runs.
-template <int C>
-__device__ __forceinline__ int group_runs(const int* key, int n, int* perm, int* rs, int* rk, int zero) {
+// 4 n entries.  Returns the number of runs.  Every lane places its own point:
+// a run's place is the sum of the padded lengths of the runs before it, a scan
+// over the lanes that lead one (a loop over the leaders cost five times the
+// instructions at ten runs).
+template <int C, class P, class R>
+__device__ __forceinline__ int group_runs(const int* key, int n, P* perm, R* rs, int* rk, int zero) {
     const int lane = threadIdx.x & 31;
     const unsigned below = (1u << lane) - 1u;
     int pos = 0, r = 0;
@@ -94,24 +97,28 @@ __device__ __forceinline__ int group_runs(const int* key, int n, int* perm, int*
         const int q = lane + 32 * j;
         const int k = q < n ? key[q] : -1;
         const unsigned peers = __match_any_sync(0xffffffffu, k);
-        unsigned leaders = __ballot_sync(0xffffffffu, k >= 0 && (peers & below) == 0u);
-        while (leaders) {
-            const int l = __ffs(leaders) - 1;
-            leaders &= leaders - 1u;
-            const unsigned grp = __shfl_sync(0xffffffffu, peers, l);
-            const int kl = __shfl_sync(0xffffffffu, k, l);
-            const int cnt = __popc(grp), padded = (cnt + 3) & ~3;
-            if ((grp >> lane) & 1u) perm[pos + __popc(grp & below)] = q;
-            if (lane < padded - cnt) perm[pos + cnt + lane] = zero;
-            if (lane == 0) {
-                rs[r] = pos;
-                rk[r] = kl;
-            }
-            pos += padded;
-            ++r;
+        const int cnt = __popc(peers), padded = (cnt + 3) & ~3;
+        const bool leads = k >= 0 && (peers & below) == 0u;
+        const unsigned leaders = __ballot_sync(0xffffffffu, leads);
+        int end = leads ? padded : 0;  // inclusive sum over the lanes
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, end, d);
+            if (lane >= d) end += v;
         }
+        // the leader's lane has summed its own run too
+        const int start = pos + __shfl_sync(0xffffffffu, end - padded, __ffs(peers) - 1);
+        if (k >= 0) perm[start + __popc(peers & below)] = P(q);
+        if (leads) {
+            for (int t = cnt; t < padded; ++t) perm[start + t] = P(zero);
+            const int mine = r + __popc(leaders & below);
+            rs[mine] = R(start);
+            rk[mine] = k;
+        }
+        pos += __shfl_sync(0xffffffffu, end, 31);
+        r += __popc(leaders);
     }
-    if (lane == 0) rs[r] = pos;
+    if (lane == 0) rs[r] = R(pos);
     __syncwarp();
     return r;
 }
@@ -134,21 +141,21 @@ __device__ __forceinline__ void mma884(double d[2], double a, double b) {
 // box.  Row `zero` (index C) of wx/wy/wz and f must be all zero; perm, rs and
 // rk are group_runs' scratch.  Touch: entries whose run sum is zero are left as
 // they are (a box that marks its untouched entries).
-template <int C, bool Touch = false>
+template <int C, bool Touch = false, class P, class R>
 __device__ __forceinline__ void spread_runs_mma(double* box, const int* key, const double* f, const double* wx,
                                                 const double* wy, const double* wz, int n, int sx, int sy,
-                                                int* perm, int* rs, int* rk) {
+                                                P* perm, R* rs, int* rk) {
     const int lane = threadIdx.x & 31;
     const int runs = group_runs<C>(key, n, perm, rs, rk, C);
     const int slot = lane & 3, row = lane >> 2;     // A: x offset `row`, point `slot`
     const int jb = lane >> 4, kb = (lane >> 2) & 3;  // B column lane/4 = (j, k) = (jb [+2], kb)
     const int ax = row & 3;
     for (int r = 0; r < runs; ++r) {
-        const int s0 = rs[r], e0 = rs[r + 1], K = rk[r];
+        const int s0 = int(rs[r]), e0 = int(rs[r + 1]), K = rk[r];
         double d0[2] = {0.0, 0.0}, d1[2] = {0.0, 0.0};
 #pragma unroll 2
         for (int b = s0 + slot; b < e0; b += 4) {
-            const int q = perm[b];
+            const int q = int(perm[b]);
             const int qa = row < 4 ? q : C;
             const double a = wx[qa * 12 + ax];
             const double fz = f[q] * wz[q * 12 + kb];
@@ -170,13 +177,33 @@ __device__ __forceinline__ void spread_runs_mma(double* box, const int* key, con
 
 // The element spread of one component: the FP64 tensor-core form for double,
 // the register-run form otherwise.
-template <class T, int C>
+template <class T, int C, class P, class R>
 __device__ __forceinline__ void spread_element(T* box, const int* key, const T* f, const T* wx, const T* wy,
-                                               const T* wz, int n, int sx, int sy, int* perm, int* rs, int* rk) {
+                                               const T* wz, int n, int sx, int sy, P* perm, R* rs, int* rk) {
     if constexpr (sizeof(T) == 8)
         spread_runs_mma<C>(box, key, f, wx, wy, wz, n, sx, sy, perm, rs, rk);
     else
         spread_runs<T, C>(box, key, f, wx, wy, wz, n, sx, sy);
+}
+
+// Row q of a basis table (NPC values, NPC even), by pairs where the table lies
+// on a pair's boundary: the lanes' rows are NPC values apart, so every load of
+// a warp touches a sector per lane and half as many loads halve the L1's work.
+template <class T, int NPC>
+__device__ __forceinline__ void basis_row(const T* __restrict__ N, int64_t q, T out[NPC]) {
+    using P = typename std::conditional<sizeof(T) == 8, double2, float2>::type;
+    if (reinterpret_cast<uintptr_t>(N) % sizeof(P) == 0) {
+        const P* row = reinterpret_cast<const P*>(N + q * NPC);
+#pragma unroll
+        for (int a = 0; a < NPC / 2; ++a) {
+            const P v = row[a];
+            out[2 * a] = v.x;
+            out[2 * a + 1] = v.y;
+        }
+    } else {
+#pragma unroll
+        for (int a = 0; a < NPC; ++a) out[a] = N[q * NPC + a];
+    }
 }
 
 // ------------------------------------------------------------------ gather
