@@ -124,6 +124,10 @@ _SIGNATURES = {
                                  c_void_p, c_void_p, c_int32, c_void_p],
     'afsi_b200_compact_gather3': [c_void_p] * 5 + [c_int64] * 4 + [c_void_p, c_void_p, c_int32, c_void_p],
     'afsi_b200_compact_spread3': [c_void_p] * 3 + [c_int64] * 4 + [c_double] + [c_void_p] * 4 + [c_int32, c_void_p],
+    'afsi_b200_compact_density': [c_void_p, c_int64, c_double, c_int32, c_void_p, c_void_p],
+    'afsi_b200_compact_binned_bytes': [c_int64] * 4,
+    'afsi_b200_compact_spread3_binned': [c_void_p] * 3 + [c_int64] * 4 + [c_double] + [c_void_p] * 4 +
+                                        [c_int64, c_void_p, c_int32, c_void_p],
     'afsi_b200_indexed_gather2': [c_void_p, c_void_p, c_int64, c_int64] + [c_void_p] * 4 +
                                  [c_int64, c_void_p, c_void_p, c_int32, c_void_p],
     'afsi_b200_indexed_spread2': [c_void_p, c_int64] + [c_void_p] * 4 + [c_int64] * 3 + [c_double] + [c_void_p] * 3 +
@@ -224,7 +228,8 @@ _SIGNATURES = {
     'afsi_b200_pcg_graph_launch': [c_void_p, c_void_p],
     'afsi_b200_pcg_graph_destroy': [c_void_p],
 }
-_RESTYPES = {'afsi_b200_last_error': ctypes.c_char_p, 'afsi_b200_mg_scratch_bytes': ctypes.c_int64,
+_RESTYPES = {'afsi_b200_last_error': ctypes.c_char_p, 'afsi_b200_compact_binned_bytes': ctypes.c_int64,
+             'afsi_b200_mg_scratch_bytes': ctypes.c_int64,
              'afsi_b200_mg_batch_table_bytes': ctypes.c_int64, 'afsi_b200_batch_refine_bytes': ctypes.c_int64,
              'afsi_b200_batch_refine_state_offset': ctypes.c_int64,
              'afsi_b200_stokes_packed_size': ctypes.c_int64,

@@ -161,6 +161,25 @@ def _component_tables(grid, values, stencil, like):
     return base, phi
 
 
+# The binned spread wins from about twelve points per occupied cell (and some
+# ten thousand points) on.  One B200, binned against plain, spread alone with its
+# launches: a shell of 400,000 points on 64^3 (50 per cell) 178 against 348 us in
+# FP64 and 213 against 244 in FP32, of 100,000 (12 per cell) 91 against 93, of
+# 60,000 on 32^3 (30 per cell) 76 against 104; 400,000 points all over 64^3 (1.5 per
+# cell) 249 against 192, 30,000 on 32^3 79 against 52.  How many share a cell is
+# measured once, when the points are binned, and read with the support flag.
+_BINNED_POINTS = 60000
+_BINNED_PER_CELL = 12.
+_DENSE_BIT = 1 << 30
+
+
+def _binned_bytes(grid, stencil, points, phi):
+    """Scratch of the binned spread where it is the faster form, else 0."""
+    if points < _BINNED_POINTS or not getattr(stencil, 'dense', False) or phi.data_ptr() % 16:
+        return 0
+    return max(int(_lib.load().afsi_b200_compact_binned_bytes(points, *grid.shape)), 0)
+
+
 def compact_gather(grid, velocity, stencil):
     require_cuda(velocity[0])
     tables = _component_tables(grid, velocity, stencil, velocity[0]) if len(velocity) == 3 else None
@@ -184,6 +203,13 @@ def compact_spread(grid, force, stencil):
         base, phi = tables
         force = force.contiguous()
         fields = tuple(torch.empty(grid.face_shape(c), device=force.device, dtype=force.dtype) for c in range(3))
+        scratch = _binned_bytes(grid, stencil, base.shape[1], phi)
+        if scratch > 0:
+            work = torch.empty(scratch, device=force.device, dtype=torch.uint8)
+            call('afsi_b200_compact_spread3_binned', ptr(force), ptr(base), ptr(phi), base.shape[1], *grid.shape,
+                 float(grid.volume), *(ptr(f) for f in fields), ptr(work), scratch,
+                 ptr(_lib.status_word(force.device)), dtype_code(force.dtype), stream(force.device))
+            return fields
         call('afsi_b200_compact_spread3', ptr(force), ptr(base), ptr(phi), base.shape[1], *grid.shape,
              float(grid.volume), *(ptr(f) for f in fields), ptr(_lib.status_word(force.device)),
              dtype_code(force.dtype), stream(force.device))
@@ -203,6 +229,7 @@ class CompactStencil:
     base: torch.Tensor
     phi: torch.Tensor
     layout: str = 'component'
+    dense: bool = False  # many points share a cell: the spread bins them first
 
     @property
     def storage_bytes(self):
@@ -245,10 +272,19 @@ def compact_prepare(grid, points, *, layout='component', phi_form='clamped', che
          _lib.doubles(grid.spacing), _lib.doubles(grid.origin), _lib.int64s(grid.shape),
          _lib.PHI_RADICAL if phi_form == 'radical' else _lib.PHI_CLAMPED, ptr(base), ptr(phi), ptr(word),
          dtype_code(points.dtype), stream(points.device))
-    if check_support and P and int(word.item()) & _lib.FLAG_SUPPORT:
-        word.zero_()
-        raise ValueError('MAC IB support reaches a wall or is nonfinite; enlarge/refine the fluid box')
-    return CompactStencil(base, phi, layout)
+    dense = False
+    if check_support and P:
+        ask = layout == 'component' and P >= _BINNED_POINTS
+        if ask:
+            call('afsi_b200_compact_density', ptr(base), P, _BINNED_PER_CELL, _DENSE_BIT, ptr(word),
+                 stream(points.device))
+        value = int(word.item())
+        dense = bool(value & _DENSE_BIT)
+        if dense or value & _lib.FLAG_SUPPORT:
+            word.zero_()
+        if value & _lib.FLAG_SUPPORT:
+            raise ValueError('MAC IB support reaches a wall or is nonfinite; enlarge/refine the fluid box')
+    return CompactStencil(base, phi, layout, dense)
 
 
 @dataclass(frozen=True)

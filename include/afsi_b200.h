@@ -309,6 +309,18 @@ int32_t afsi_b200_compact_gather3(const void* u0, const void* u1, const void* u2
 int32_t afsi_b200_compact_spread3(const void* force, const int64_t* base, const void* phi, int64_t points,
     int64_t nx, int64_t ny, int64_t nz, double volume, void* u0, void* u1, void* u2, int32_t* status,
     int32_t dtype, afsi_stream_t stream);
+/* spread3 with the points binned by lattice cell first: several points of a
+ * cell or tile are summed on chip and reduced into a face once.  Same
+ * arguments; phi 16-byte aligned, points < 2^31 - 1, and `scratch` of at least
+ * compact_binned_bytes (-1: sizes that only spread3 takes).  */
+/* compact_density sets `bit` of the status word when the points, by a sample,
+ * hold more than per_cell of them per occupied cell of component 0's base. */
+int32_t afsi_b200_compact_density(const int64_t* base, int64_t points, double per_cell, int32_t bit,
+    int32_t* status, afsi_stream_t stream);
+int64_t afsi_b200_compact_binned_bytes(int64_t points, int64_t nx, int64_t ny, int64_t nz);
+int32_t afsi_b200_compact_spread3_binned(const void* force, const int64_t* base, const void* phi, int64_t points,
+    int64_t nx, int64_t ny, int64_t nz, double volume, void* u0, void* u1, void* u2, void* scratch,
+    int64_t scratch_bytes, int32_t* status, int32_t dtype, afsi_stream_t stream);
 /* Both components of a 2D channel transfer in one launch, 16 taps per point:
  * u (nu values) and v (nv), point values (points, 2) out of the gather, and
  * `stride` >= 2 values per point into the spread, which clears u and v first. */
