@@ -5,7 +5,7 @@
 // component, at the L2's 110 G sector reductions/s.  Where many markers share a
 // lattice cell most of those reductions meet in the same faces.  Here the points
 // are ordered by 4x4x4-cell tile and cell (a count per cell, a scan, a place per
-// point), a warp takes 64 consecutive points and sums each component into a box
+// point), a warp takes 32 consecutive points and sums each component into a box
 // in shared memory, and each face of the box is reduced once.  A box that covers
 // all of the warp's points is used where it fits, else the points go tile by
 // tile: a tile's box is at most 8x8x8 faces (four cells, one more where the
@@ -14,13 +14,14 @@
 // cores, runs.cuh), others are added one by one; few points of a tile are reduced
 // directly.
 //
-// What bounds it is latency at 16 warps per SM (128 registers, 14 KB of shared
+// What bounds it is latency at 20 warps per SM (96 registers, 9.5 KB of shared
 // memory a warp), first of all the scattered reads of the table rows.  Lanes
 // therefore read whole rows together (cp.async, 16 bytes each), the bases and
 // forces of all components are requested at once, and the next component's rows
-// are in flight while a box is flushed: 186 -> 138 us.  400,000 markers of a shell
-// on 64^3 (50 per cell), FP64, one B200: 305 us plain, 138 us and 36 us of binning
-// and clearing here.  The caller chooses the form by the cloud's density
+// are in flight while a box is flushed: 186 -> 138 us; 32 points per warp at 20
+// warps instead of 64 at 16: 123 us (24 warps: 127).  400,000 markers of a shell on
+// 64^3 (50 per cell), FP64, one B200: 305 us plain, 123 us and 36 us of binning and
+// clearing here.  The caller chooses the form by the cloud's density
 // (bin_density_kernel, cuda_ib.compact_spread).
 #include <cub/device/device_scan.cuh>
 #include <climits>
@@ -32,7 +33,7 @@ namespace afsi {
 namespace {
 
 constexpr int kBinWarps = 4;
-constexpr int kBinPoints = 64;    // points per warp
+constexpr int kBinPoints = 32;    // points per warp
 constexpr int kBinCap = 608;      // padded 8x8x8 box
 constexpr int kBinMerge = 3;      // points per run from which the runs are summed first
 constexpr int kBinOut = 0xffff;
@@ -166,7 +167,7 @@ __device__ __forceinline__ void bin_points(T* box, const int* at, const T* f, co
 }
 
 template <class T>
-__global__ void __launch_bounds__(kBinWarps * 32, 4) bin_spread_kernel(
+__global__ void __launch_bounds__(kBinWarps * 32, 5) bin_spread_kernel(
     const T* __restrict__ force, const int64_t* __restrict__ base, const T* __restrict__ phi, int64_t points,
     const int32_t* __restrict__ order, BinGrid g, T volume, T inv_volume,
     T* __restrict__ u0, T* __restrict__ u1, T* __restrict__ u2, int32_t* status) {
@@ -227,16 +228,17 @@ __global__ void __launch_bounds__(kBinWarps * 32, 4) bin_spread_kernel(
         for (int j = 0; j < J; ++j) left[j] = live[j];
         bool whole = true, fetched = c == 2;  // the next component's rows
         while (true) {
-            const unsigned m0 = __ballot_sync(0xffffffffu, left[0]), m1 = __ballot_sync(0xffffffffu, left[1]);
-            if (!(m0 | m1)) {
+            bool some = false;
+            unsigned now = 0;  // the tile of a point that is left
+#pragma unroll
+            for (int j = 0; j < J; ++j) {
+                const unsigned m = __ballot_sync(0xffffffffu, left[j]);
+                if (m) now = __shfl_sync(0xffffffffu, tile[j], __ffs(m) - 1);
+                some = some || m;
+            }
+            if (!some) {
                 if (!fetched) bin_fetch_rows(s, phi, points, c + 1, n);  // no point of this component
                 break;
-            }
-            unsigned now = 0;
-            if (!whole) {
-                const unsigned t0 = __shfl_sync(0xffffffffu, tile[0], m0 ? __ffs(m0) - 1 : 0);
-                const unsigned t1 = __shfl_sync(0xffffffffu, tile[1], m1 ? __ffs(m1) - 1 : 0);
-                now = m0 ? t0 : t1;
             }
             bool take[J];
             int mn[3] = {INT_MAX, INT_MAX, INT_MAX}, mx[3] = {INT_MIN, INT_MIN, INT_MIN};
@@ -270,9 +272,15 @@ __global__ void __launch_bounds__(kBinWarps * 32, 4) bin_spread_kernel(
                 for (int j = 0; j < J; ++j) left[j] = live[j];
                 continue;
             }
-            const bool fetch = !fetched && !__any_sync(0xffffffffu, left[0] || left[1]);
+            bool mine = false;
+            int count = 0;
+#pragma unroll
+            for (int j = 0; j < J; ++j) {
+                mine = mine || left[j];
+                count += __popc(__ballot_sync(0xffffffffu, take[j]));
+            }
+            const bool fetch = !fetched && !__any_sync(0xffffffffu, mine);
             fetched = fetched || fetch;
-            const int count = __popc(__ballot_sync(0xffffffffu, take[0])) + __popc(__ballot_sync(0xffffffffu, take[1]));
             if (fits && count >= kBinFew) {
                 const int size = ex * sx;
                 for (int t = lane; t < size; t += 32) s.box[t] = T(0);
@@ -324,11 +332,11 @@ __global__ void __launch_bounds__(kBinWarps * 32, 4) bin_spread_kernel(
                         int src = 0;
                         unsigned rest = todo;
                         for (int k = 0; k < (lane >> 2) && rest; ++k) rest &= rest - 1;
-                        const bool mine = rest != 0;
-                        src = mine ? __ffs(rest) - 1 : 0;
+                        const bool has = rest != 0;
+                        src = has ? __ffs(rest) - 1 : 0;
                         const int bx = __shfl_sync(0xffffffffu, b[j][0], src), by = __shfl_sync(0xffffffffu, b[j][1], src),
                                   bz = __shfl_sync(0xffffffffu, b[j][2], src);
-                        if (mine) {
+                        if (has) {
                             const T* w = s.w + (src + 32 * j) * 12;
                             const int k = lane & 3;
                             const T fz = s.f[src + 32 * j] * w[8 + k];
