@@ -50,7 +50,7 @@ __device__ __forceinline__ int bin_extent(const BinGrid& g, int c, int a) {
 }
 
 __device__ __forceinline__ unsigned bin_key(int64_t x, int64_t y, int64_t z, const BinGrid& g) {
-    if (!(x >= 0 && y >= 0 && z >= 0 && x + 3 <= g.nx && y + 3 < g.ny && z + 3 < g.nz)) return g.none;
+    if (!(x >= 0 && y >= 0 && z >= 0 && x <= g.nx - 3 && y < g.ny - 3 && z < g.nz - 3)) return g.none;
     const int ix = int(x), iy = int(y), iz = int(z);
     return unsigned(((ix >> 2) * g.t1 + (iy >> 2)) * g.t2 + (iz >> 2)) * 64u +
            unsigned(((ix & 3) << 4) | ((iy & 3) << 2) | (iz & 3));

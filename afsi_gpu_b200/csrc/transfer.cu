@@ -14,7 +14,8 @@
 // components run in one launch (grid y), reading the force and writing the
 // velocities in their (P, 3) layout.  400,000 markers on 64^3, FP64, one B200:
 // spread 668 -> 305 us (110 G sector reductions/s, the L2's rate either way),
-// gather 172 -> 81 us.  The 2D pair (20,000 markers, 256 x 64) is bound by
+// gather 172 -> 81 us.  Clouds with many points per cell take the binned spread
+// (compact_bins.cu).  The 2D pair (20,000 markers, 256 x 64) is bound by
 // launches: 29 -> 8 us of spread and 12 device operations -> 7 for a transfer.
 #include <cmath>
 #include "common.cuh"
