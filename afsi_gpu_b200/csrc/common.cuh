@@ -102,6 +102,11 @@ __device__ __forceinline__ T exact_reciprocal(T v) {
     }
 }
 
+// The four faces of a support that starts at b lie inside [0, n).  Any table
+// entry: points without a support check bin to the ends of the 64-bit range,
+// where b + 3 wraps.
+__host__ __device__ __forceinline__ bool support_inside(int64_t b, int64_t n) { return b >= 0 && b <= n - 4; }
+
 __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_enter() {

@@ -114,7 +114,8 @@ __global__ void __launch_bounds__(256) rows_boxes_kernel(const int64_t* __restri
 #pragma unroll
             for (int a = 0; a < 3; ++a) {
                 const int l = a != c;
-                const bool in = mn[l][a] >= 0 && mx[l][a] + 4 <= face_n(g, c, a) && mx[l][a] - mn[l][a] + 4 <= kMaxExt;
+                const bool in = mn[l][a] >= 0 && support_inside(mx[l][a], face_n(g, c, a)) &&
+                                mx[l][a] - mn[l][a] + 4 <= kMaxExt;
                 ok = ok && in;
                 lo[a] = in ? int(mn[l][a]) : 0;
                 hi[a] = in ? int(mx[l][a]) : 0;

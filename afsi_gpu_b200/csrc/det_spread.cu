@@ -66,7 +66,7 @@ __global__ void det_keys_kernel(const int64_t* __restrict__ base, DetGrid g, int
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
             o[a] = base[det_row(g.total, p, c, a)];
-            inside = inside && o[a] >= 0 && o[a] + 3 < face_extent(g, c, a);
+            inside = inside && support_inside(o[a], face_extent(g, c, a));
         }
         if (!inside) flag(status, AFSI_FLAG_INDEX);
         keys[p] = uint32_t(inside ? (o[0] / kTile * tiles_along(g, c, 1) + o[1] / kTile) * tiles_along(g, c, 2) +

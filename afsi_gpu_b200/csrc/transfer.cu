@@ -100,7 +100,7 @@ __global__ void __launch_bounds__(256) indexed_pair_kernel(Pair2D<T> a, int64_t 
 
 // False (and the caller flags) if the 4x4x4 box leaves [0,n).
 __device__ __forceinline__ bool box_inside(int64_t bx, int64_t by, int64_t bz, int64_t nx, int64_t ny, int64_t nz) {
-    return bx >= 0 && by >= 0 && bz >= 0 && bx + 3 < nx && by + 3 < ny && bz + 3 < nz;
+    return support_inside(bx, nx) && support_inside(by, ny) && support_inside(bz, nz);
 }
 
 // Components of one launch: face arrays and their dims, tables of the first
