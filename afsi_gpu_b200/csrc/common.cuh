@@ -5,6 +5,7 @@
 // source rounds twice, as in the reference CPU/Triton arithmetic; kernels
 // that want a fused multiply-add say so with fma().
 #pragma once
+#include <atomic>
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <math.h>
@@ -14,6 +15,47 @@ namespace afsi {
 
 int32_t fail(int32_t code, const char* fmt, ...);
 int32_t launched(const char* what);  // AFSI_OK or AFSI_ERR_CUDA after a launch
+
+// A number found once per device (-1: not found yet, or a device beyond the
+// list, for which it is found on every call).
+class PerDevice {
+public:
+    int get() const {
+        const int d = device();
+        return d < 0 ? -1 : value_[d].load(std::memory_order_acquire) - 1;
+    }
+    void set(int v) {
+        const int d = device();
+        if (d >= 0) value_[d].store(v + 1, std::memory_order_release);
+    }
+
+private:
+    static constexpr int kDevices = 64;
+    static int device() {
+        int d = -1;
+        return cudaGetDevice(&d) == cudaSuccess && d < kDevices ? d : -1;
+    }
+    std::atomic<int> value_[kDevices] = {};
+};
+
+// Lets Kernel take `bytes` of dynamic shared memory on the current device, the
+// same number on every call.  Function attributes belong to a device, so this
+// stands before every launch that needs more than the default, and the attribute
+// is set on each device's first (setting it every time cost some 2 us per launch).  It touches
+// no stream and may be called during a capture.
+template <auto Kernel>
+int32_t allow_shared(const char* what, size_t bytes) {
+    static PerDevice known;
+    if (known.get() == int(bytes)) return AFSI_OK;
+    const cudaError_t err = cudaFuncSetAttribute(reinterpret_cast<const void*>(Kernel),
+                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes));
+    if (err != cudaSuccess) {
+        cudaGetLastError();
+        return fail(AFSI_ERR_CUDA, "%s: shared memory: %s", what, cudaGetErrorString(err));
+    }
+    known.set(int(bytes));
+    return AFSI_OK;
+}
 
 inline unsigned blocks_for(int64_t n, int threads) {
     return static_cast<unsigned>((n + threads - 1) / threads);

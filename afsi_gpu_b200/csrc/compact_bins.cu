@@ -423,9 +423,7 @@ extern "C" int32_t afsi_b200_compact_spread3_binned(const void* force, const int
         int ex = 0;
         const T inv = std::frexp(double(vol), &ex) == 0.5 && std::isnormal(T(1) / vol) ? T(1) / vol : T(0);
         const size_t smem = sizeof(BinStage<T>) * kBinWarps;
-        if (cudaFuncSetAttribute(bin_spread_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) !=
-            cudaSuccess)
-            return fail(AFSI_ERR_CUDA, "binned spread shared memory: %s", cudaGetErrorString(cudaGetLastError()));
+        if ((rc = allow_shared<bin_spread_kernel<T>>("compact_spread3_binned", smem))) return rc;
         const int64_t warps = (points + kBinPoints - 1) / kBinPoints;
         bin_spread_kernel<T><<<blocks_for(warps, kBinWarps), kBinWarps * 32, smem, stream>>>(
             static_cast<const T*>(force), base, static_cast<const T*>(phi), points, order, g, vol, inv,

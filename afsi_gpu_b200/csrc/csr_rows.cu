@@ -541,9 +541,7 @@ extern "C" int32_t afsi_b200_p1_rows_fill(const int64_t* base, const void* phi, 
             gr.nq[k] = int(groups[k].nq);
         }
         const size_t smem = fill_smem<T>(box_cap);
-        if (cudaFuncSetAttribute(rows_fill_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kRowsSmem) + 4096) !=
-            cudaSuccess)
-            return fail(AFSI_ERR_CUDA, "row fill shared memory: %s", cudaGetErrorString(cudaGetLastError()));
+        if ((rc = allow_shared<rows_fill_kernel<T>>("p1_rows_fill", kRowsSmem + 4096))) return rc;
         const int64_t want = (nodes + kRowsWarps - 1) / kRowsWarps;
         rows_fill_kernel<T><<<dim3(unsigned(std::min<int64_t>(want, 1 << 20)), 3), kRowsWarps * 32, smem, stream>>>(
             base, static_cast<const T*>(phi), total, gr, start, slots, int(nodes),

@@ -368,11 +368,7 @@ extern "C" int32_t afsi_b200_det_spread(const void* force, const int64_t* base, 
     void* fields[3] = {u0, u1, u2};
     AFSI_DISPATCH(dtype, {
         const size_t smem = size_t(kDetWarps) * kBox * sizeof(T) + kChunkRows * sizeof(int32_t);
-        static bool configured = false;  // once per instantiation, before any graph capture of it
-        if (!configured) {
-            cudaFuncSetAttribute(det_tile_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-            configured = true;
-        }
+        if ((rc = allow_shared<det_tile_kernel<T>>("det_spread", smem))) return rc;
         for (int c = 0; c < 3; ++c) {
             const int64_t tiles = tile_count(g, c);
             T* scratch = reinterpret_cast<T*>(b + L.scratch);

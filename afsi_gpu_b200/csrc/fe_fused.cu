@@ -1267,12 +1267,7 @@ extern "C" int32_t afsi_b200_fe_fused_spread(int32_t nodes_per_cell, const void*
         const int G = elements_per_warp(elements, nq, NPC, kMPoints);
         if (G > 1) {
             const size_t multi = sizeof(MStage<TP, T, NPC>) * kMWarps;
-            static bool multi_configured = false;  // once per instantiation, before any graph capture of it
-            if (!multi_configured) {
-                cudaFuncSetAttribute(fused_spread_multi_kernel<TP, T, NPC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     int(multi));
-                multi_configured = true;
-            }
+            if ((rc = allow_shared<fused_spread_multi_kernel<TP, T, NPC>>("fused_spread_multi", multi))) return rc;
             const T vol = T(volume);
             int ex = 0;
             const bool pow2 = std::frexp(double(vol), &ex) == 0.5 && std::isnormal(T(1) / vol);
@@ -1285,12 +1280,7 @@ extern "C" int32_t afsi_b200_fe_fused_spread(int32_t nodes_per_cell, const void*
             return launched("fused_spread_multi");
         }
         const size_t smem = sizeof(FStage<TP, T, NPC>) * kFWarps;
-        static bool configured = false;  // once per instantiation, before any graph capture of it
-        if (!configured) {
-            cudaFuncSetAttribute(fused_spread_kernel<TP, T, NPC, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 int(smem));
-            configured = true;
-        }
+        if ((rc = allow_shared<fused_spread_kernel<TP, T, NPC, 0>>("fused_spread", smem))) return rc;
         fused_spread_kernel<TP, T, NPC, 0><<<fused_blocks(elements, kFWarps), kFWarps * 32, smem, s>>>(
             static_cast<const TP*>(x), cells, static_cast<const TP*>(N_pos), static_cast<const T*>(N),
             static_cast<const T*>(W), static_cast<const T*>(value), make_geo<TP>(origin, spacing, limits),
@@ -1354,14 +1344,8 @@ extern "C" int32_t afsi_b200_fe_det_spread(int32_t nodes_per_cell, const void* x
         const Geo<TP> geo = make_geo<TP>(origin, spacing, limits);
         const size_t smem1 = sizeof(FStage<TP, T, NPC, kFBoxCap>) * kFWarps;
         const size_t smem2 = sizeof(FStage<TP, T, NPC, kDetBoxCap>) * kFWarps;
-        static bool configured = false;  // once per instantiation, before any graph capture of it
-        if (!configured) {
-            cudaFuncSetAttribute(fused_spread_kernel<TP, T, NPC, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 int(smem1));
-            cudaFuncSetAttribute(fused_spread_kernel<TP, T, NPC, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 int(smem2));
-            configured = true;
-        }
+        if ((rc = allow_shared<fused_spread_kernel<TP, T, NPC, 1>>("fe_det_spread boxes", smem1))) return rc;
+        if ((rc = allow_shared<fused_spread_kernel<TP, T, NPC, 2>>("fe_det_spread large boxes", smem2))) return rc;
         fused_spread_kernel<TP, T, NPC, 1><<<fused_blocks(elements, kFWarps), kFWarps * 32, smem1, s>>>(
             static_cast<const TP*>(x), cells, static_cast<const TP*>(N_pos), static_cast<const T*>(N),
             static_cast<const T*>(W), static_cast<const T*>(value), geo, static_cast<T*>(u0), static_cast<T*>(u1),
@@ -1410,12 +1394,7 @@ static int32_t fused_gather(int32_t nodes_per_cell, const void* x, int64_t nodes
         const int G = elements_per_warp(elements, nq, NPC, kMGPoints);
         if (G > 1) {
             const size_t multi = sizeof(MGStage<TP, T, NPC>) * kMWarps;
-            static bool multi_configured = false;  // once per instantiation, before any graph capture of it
-            if (!multi_configured) {
-                cudaFuncSetAttribute(fused_gather_multi_kernel<TP, T, NPC, Local>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, int(multi));
-                multi_configured = true;
-            }
+            if ((rc = allow_shared<fused_gather_multi_kernel<TP, T, NPC, Local>>("fused_gather_multi", multi))) return rc;
             fused_gather_multi_kernel<TP, T, NPC, Local>
                 <<<fused_blocks((elements + G - 1) / G, kMWarps), kMWarps * 32, multi, s>>>(
                     static_cast<const T*>(u0), static_cast<const T*>(u1), static_cast<const T*>(u2),
@@ -1424,12 +1403,7 @@ static int32_t fused_gather(int32_t nodes_per_cell, const void* x, int64_t nodes
             return launched(Local ? "fused_gather_local_multi" : "fused_gather_multi");
         }
         const size_t smem = sizeof(FGStage<TP, T, NPC>) * kGWarps;
-        static bool configured = false;  // once per instantiation, before any graph capture of it
-        if (!configured) {
-            cudaFuncSetAttribute(fused_gather_kernel<TP, T, NPC, Local>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 int(smem));
-            configured = true;
-        }
+        if ((rc = allow_shared<fused_gather_kernel<TP, T, NPC, Local>>("fused_gather", smem))) return rc;
         fused_gather_kernel<TP, T, NPC, Local><<<fused_blocks(elements, kGWarps), kGWarps * 32, smem, s>>>(
             static_cast<const T*>(u0), static_cast<const T*>(u1), static_cast<const T*>(u2),
             static_cast<const TP*>(x), cells, static_cast<const TP*>(N_pos), static_cast<const T*>(N),

@@ -865,11 +865,8 @@ struct Runner {
         int64_t cells = 0;
         for (int k = l; k < plan->levels; ++k) cells += lv[k].n;
         const size_t bytes = (size_t(cells) * 3 + 64 * size_t(plan->levels - l)) * sizeof(T);
-        static bool configured = false;  // once per instantiation, before any graph capture of it
-        if (!configured) {
-            cudaFuncSetAttribute(coarse_kernel<BC, T, TC>, cudaFuncAttributeMaxDynamicSharedMemorySize, 210 * 1024);
-            configured = true;
-        }
+        const int32_t rc = allow_shared<coarse_kernel<BC, T, TC>>("mg coarse block", 210 * 1024);
+        if (rc) return rc;
         *out = P(l);
         return launch_pdl("mg coarse block", coarse_kernel<BC, T, TC>, dim3(1), dim3(kCoarseThreads), bytes, stream,
                           R(l), rhs_sum, l == 0 ? P(0) : nullptr, P(l), static_cast<const TC*>(plan->coarse_inverse),
@@ -947,10 +944,11 @@ struct Runner {
     }
 
     // Largest cluster (16, else 8) that this device runs with 1024-thread
-    // CTAs and 200 KB of shared memory each; 0 if none.  Queried once per
-    // instantiation, on the first (uncaptured) run.
+    // CTAs and 200 KB of shared memory each; 0 if none.  Queried, and the kernel
+    // configured, once per instantiation and device, on the first (uncaptured) run.
     static int cluster_capacity() {
-        static int capacity = -1;
+        static PerDevice known;
+        int capacity = known.get();
         if constexpr (is3d(BC)) {
             if (capacity < 0) {
                 capacity = 0;
@@ -980,6 +978,7 @@ struct Runner {
                     }
                     cudaGetLastError();
                 }
+                known.set(capacity);
             }
         }
         return capacity < 0 ? 0 : capacity;
@@ -1212,12 +1211,8 @@ struct RbRunner {
         int64_t cells = 0;
         for (int k = l; k < plan->levels; ++k) cells += lv[k].n;
         const size_t bytes = (size_t(cells) * 3 + 64 * size_t(plan->levels - l)) * sizeof(T);
-        static bool configured = false;  // once per instantiation, before any graph capture of it
-        if (!configured) {
-            cudaFuncSetAttribute(coarse_rb_kernel<BC, T, TC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 210 * 1024);
-            configured = true;
-        }
+        const int32_t rc = allow_shared<coarse_rb_kernel<BC, T, TC>>("mg red-black coarse block", 210 * 1024);
+        if (rc) return rc;
         return launch_pdl("mg red-black coarse block", coarse_rb_kernel<BC, T, TC>, dim3(1), dim3(kCoarseThreads),
                           bytes, stream, static_cast<const T*>(R(l)), static_cast<const T*>(l == 0 ? P(0) : nullptr),
                           P(l), static_cast<const TC*>(plan->coarse_inverse), cl, plan->smooth);
@@ -2344,12 +2339,7 @@ int32_t batch_cycles(const afsi_mg_plan* const* plans, int count, const unsigned
     BatchLayout lay;
     int32_t rc = batch_table<T, TC>(plans, count, nullptr, lay, nullptr);
     if (rc) return rc;
-    static bool configured = false;  // once per instantiation, before any graph capture of it
-    if (!configured) {
-        cudaFuncSetAttribute(batch_coarse_kernel<BC, T, TC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             210 * 1024);
-        configured = true;
-    }
+    if ((rc = allow_shared<batch_coarse_kernel<BC, T, TC>>("mg batch coarse block", 210 * 1024))) return rc;
     const int smooth = plans[0]->smooth;
     auto lv = [&](int d) { return reinterpret_cast<const BatchLevel<T>*>(table + lay.level_off[d]); };
     auto ml = [&](int d) { return reinterpret_cast<const uint32_t*>(table + lay.map_l_off[d]); };
@@ -2429,10 +2419,13 @@ int32_t batch_persistent(const afsi_mg_plan* const* plans, int count, const unsi
     a.gs.slot = reinterpret_cast<double*>(b + 64);
     a.gs.partial = reinterpret_cast<double*>(b + 64 + 8 * (AFSI_MG_MAX_LEVELS * 3 + 8));
     auto kernel = batch_persistent_kernel<BC, T, TC>;
-    static int per_sm = -1;  // once per instantiation, before any graph capture of it
+    static PerDevice known;  // blocks per SM; found and the kernel configured before any graph capture of it
+    int per_sm = known.get();
     if (per_sm < 0) {
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 210 * 1024);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kBatchPThreads, 200 * 1024);
+        if ((rc = allow_shared<batch_persistent_kernel<BC, T, TC>>("mg batch persistent", 210 * 1024))) return rc;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kBatchPThreads, 200 * 1024) != cudaSuccess)
+            return fail(AFSI_ERR_CUDA, "persistent batched V-cycles: %s", cudaGetErrorString(cudaGetLastError()));
+        known.set(per_sm);
     }
     int device = 0, sms = 0;
     cudaGetDevice(&device);

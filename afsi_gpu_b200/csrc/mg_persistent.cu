@@ -308,11 +308,8 @@ int32_t run_persistent(const afsi_mg_plan* plan, int cycles, int solve, int chec
     a.gs.partial = reinterpret_cast<double*>(b + 64 + 8 * (kNormSlot + 8));
 
     auto kernel = mg_persistent<BC, T, TC>;
-    static bool configured = false;
-    if (!configured) {
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 210 * 1024);
-        configured = true;
-    }
+    const int32_t rc = allow_shared<mg_persistent<BC, T, TC>>("persistent multigrid", 210 * 1024);
+    if (rc) return rc;
     int device = 0, sms = 0, per_sm = 0;
     cudaGetDevice(&device);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
