@@ -170,7 +170,6 @@ def _component_tables(grid, values, stencil, like):
 # measured once, when the points are binned, and read with the support flag.
 _BINNED_POINTS = 60000
 _BINNED_PER_CELL = 12.
-_DENSE_BIT = 1 << 30
 
 
 def _binned_bytes(grid, stencil, points, phi):
@@ -268,23 +267,25 @@ def compact_prepare(grid, points, *, layout='component', phi_form='clamped', che
     word = _lib.status_word(points.device)
     if check_support:
         word.zero_()
+    # a cloud whose density is asked for has two words of its own, the support flag and the answer, read in one copy:
+    # the stream's word holds violations only, and other callers raise on any bit of it
+    ask = check_support and layout == 'component' and P >= _BINNED_POINTS
+    own = torch.zeros(2, device=points.device, dtype=torch.int32) if ask else word
     call('afsi_b200_compact_prepare', ptr(points), P, L, _lib.doubles(sum(map(list, origins), [])),
          _lib.doubles(grid.spacing), _lib.doubles(grid.origin), _lib.int64s(grid.shape),
-         _lib.PHI_RADICAL if phi_form == 'radical' else _lib.PHI_CLAMPED, ptr(base), ptr(phi), ptr(word),
+         _lib.PHI_RADICAL if phi_form == 'radical' else _lib.PHI_CLAMPED, ptr(base), ptr(phi), ptr(own),
          dtype_code(points.dtype), stream(points.device))
     dense = False
-    if check_support and P:
-        ask = layout == 'component' and P >= _BINNED_POINTS
-        if ask:
-            call('afsi_b200_compact_density', ptr(base), P, _BINNED_PER_CELL, _DENSE_BIT, ptr(word),
-                 stream(points.device))
-        value = int(word.item())
-        dense = bool(value & _DENSE_BIT)
-        if dense or value & _lib.FLAG_SUPPORT:
+    if ask:
+        call('afsi_b200_compact_density', ptr(base), P, _BINNED_PER_CELL, 1, ptr(own[1:]), stream(points.device))
+        flags, dense = own.tolist()
+    else:
+        flags = int(word.item()) if check_support and P else 0
+    if flags & _lib.FLAG_SUPPORT:
+        if not ask:
             word.zero_()
-        if value & _lib.FLAG_SUPPORT:
-            raise ValueError('MAC IB support reaches a wall or is nonfinite; enlarge/refine the fluid box')
-    return CompactStencil(base, phi, layout, dense)
+        raise ValueError('MAC IB support reaches a wall or is nonfinite; enlarge/refine the fluid box')
+    return CompactStencil(base, phi, layout, bool(dense))
 
 
 @dataclass(frozen=True)
