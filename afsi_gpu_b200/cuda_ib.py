@@ -161,20 +161,32 @@ def _component_tables(grid, values, stencil, like):
     return base, phi
 
 
-# The binned spread wins from about twelve points per occupied cell (and some
-# ten thousand points) on.  One B200, binned against plain, spread alone with its
-# launches: a shell of 400,000 points on 64^3 (50 per cell) 178 against 348 us in
-# FP64 and 213 against 244 in FP32, of 100,000 (12 per cell) 91 against 93, of
-# 60,000 on 32^3 (30 per cell) 76 against 104; 400,000 points all over 64^3 (1.5 per
-# cell) 249 against 192, 30,000 on 32^3 79 against 52.  How many share a cell is
-# measured once, when the points are binned, and read with the support flag.
+# The binned spread wins where many points share a cell.  What it saves grows with
+# the points and with how many share one; what it costs is a fixed 30 us of binning
+# and, per cell of the grid, two words that are cleared and scanned.  One B200, points
+# per occupied cell from which it is the faster form (a shell's cloud in any order,
+# both spreads with all their launches and scratch), FP64: 60,000 points 20 on 64^3 and
+# 30 on 128^3; 100,000 14 and 20; 200,000 below 12 and 14; 256^3 50 at 200,000, 15 at
+# 400,000, 4 at a million; 512^3 none up to a million (60,000: 840 against 490 us and
+# 1.1 GB of scratch).  So: 16 points per cell at 64,000 points and a fiftieth of the
+# grid's cells, fewer in proportion to the points (12 at least), and no more than 48
+# cells per point.  How many share a cell is measured once, when the points are binned,
+# and read with the support flag.
 _BINNED_POINTS = 60000
-_BINNED_PER_CELL = 12.
+
+
+def _binned_per_cell(points, shape, dtype):
+    """Points per occupied cell from which a cloud takes the binned spread, or None."""
+    cells = prod(shape)
+    if points < _BINNED_POINTS or cells > 48 * points:
+        return None
+    return max(12., 16. * (64000 + cells / 50) / points)
 
 
 def _binned_bytes(grid, stencil, points, phi):
     """Scratch of the binned spread where it is the faster form, else 0."""
-    if points < _BINNED_POINTS or not getattr(stencil, 'dense', False) or phi.data_ptr() % 16:
+    if (not getattr(stencil, 'dense', False) or phi.data_ptr() % 16
+            or _binned_per_cell(points, grid.shape, phi.dtype) is None):
         return 0
     return max(int(_lib.load().afsi_b200_compact_binned_bytes(points, *grid.shape)), 0)
 
@@ -269,7 +281,8 @@ def compact_prepare(grid, points, *, layout='component', phi_form='clamped', che
         word.zero_()
     # a cloud whose density is asked for has two words of its own, the support flag and the answer, read in one copy:
     # the stream's word holds violations only, and other callers raise on any bit of it
-    ask = check_support and layout == 'component' and P >= _BINNED_POINTS
+    per_cell = _binned_per_cell(P, grid.shape, points.dtype) if check_support and layout == 'component' else None
+    ask = per_cell is not None
     own = torch.zeros(2, device=points.device, dtype=torch.int32) if ask else word
     call('afsi_b200_compact_prepare', ptr(points), P, L, _lib.doubles(sum(map(list, origins), [])),
          _lib.doubles(grid.spacing), _lib.doubles(grid.origin), _lib.int64s(grid.shape),
@@ -277,7 +290,7 @@ def compact_prepare(grid, points, *, layout='component', phi_form='clamped', che
          dtype_code(points.dtype), stream(points.device))
     dense = False
     if ask:
-        call('afsi_b200_compact_density', ptr(base), P, _BINNED_PER_CELL, 1, ptr(own[1:]), stream(points.device))
+        call('afsi_b200_compact_density', ptr(base), P, per_cell, 1, ptr(own[1:]), stream(points.device))
         flags, dense = own.tolist()
     else:
         flags = int(word.item()) if check_support and P else 0
