@@ -277,19 +277,21 @@ def compact_prepare(grid, points, *, layout='component', phi_form='clamped', che
     base = torch.empty((L, P, 3), device=points.device, dtype=torch.int64)
     phi = torch.empty((L, P, 3, 4), device=points.device, dtype=points.dtype)
     word = _lib.status_word(points.device)
-    if check_support:
-        word.zero_()
     # a cloud whose density is asked for has two words of its own, the support flag and the answer, read in one copy:
     # the stream's word holds violations only, and other callers raise on any bit of it
     per_cell = _binned_per_cell(P, grid.shape, points.dtype) if check_support and layout == 'component' else None
     ask = per_cell is not None
-    own = torch.zeros(2, device=points.device, dtype=torch.int32) if ask else word
+    if ask:
+        own = torch.zeros(2, device=points.device, dtype=torch.int32)
+    else:
+        own = word.zero_() if check_support else word
     call('afsi_b200_compact_prepare', ptr(points), P, L, _lib.doubles(sum(map(list, origins), [])),
          _lib.doubles(grid.spacing), _lib.doubles(grid.origin), _lib.int64s(grid.shape),
          _lib.PHI_RADICAL if phi_form == 'radical' else _lib.PHI_CLAMPED, ptr(base), ptr(phi), ptr(own),
          dtype_code(points.dtype), stream(points.device))
     dense = False
     if ask:
+        word.zero_()  # as every checked prepare does; queued behind the kernel, which the host need not wait for
         call('afsi_b200_compact_density', ptr(base), P, per_cell, 1, ptr(own[1:]), stream(points.device))
         flags, dense = own.tolist()
     else:
