@@ -168,19 +168,31 @@ def _component_tables(grid, values, stencil, like):
 # both spreads with all their launches and scratch), FP64: 60,000 points 20 on 64^3 and
 # 30 on 128^3; 100,000 14 and 20; 200,000 below 12 and 14; 256^3 50 at 200,000, 15 at
 # 400,000, 4 at a million; 512^3 none up to a million (60,000: 840 against 490 us and
-# 1.1 GB of scratch).  So: 16 points per cell at 64,000 points and a fiftieth of the
-# grid's cells, fewer in proportion to the points (12 at least), and no more than 48
-# cells per point.  How many share a cell is measured once, when the points are binned,
-# and read with the support flag.
+# 1.1 GB of scratch).  In FP32 the plain form's reductions cost less and the sums on
+# chip have no tensor cores: 60,000 points 50 on 64^3 and none on 128^3; 100,000 40;
+# 200,000 22 on 64^3, 25 on 128^3, 38 on 192^3; more points 16 to 22 up to 192^3; 256^3
+# none at any.  How many share a cell is sampled once, when the points are binned
+# (bin_density_kernel), and read with the support flag; the sample counts by points, so a
+# cloud whose cells are unevenly full reads denser than its mean, this shell by a third.
+# With the lines below, over 618 clouds of 9 to 64 per cell on 32^3 to 256^3, the form
+# taken is 0.5 % slower than the faster one on average, where 12 per cell for every type
+# and grid was 7.7 % slower.
 _BINNED_POINTS = 60000
+# points at which `even` per cell break even: on the smallest grid, more up to 64^3 cells (FP32, where the plain
+# form's reductions meet less), and a fiftieth of the cells; even (in proportion to the points), the least per cell,
+# the most cells per point, the most cells
+_BINNED = {torch.float64: (64000, 0, 20., 12., 96, 1 << 62), torch.float32: (60000, 44000, 40., 26., 40, 1 << 23)}
 
 
 def _binned_per_cell(points, shape, dtype):
     """Points per occupied cell from which a cloud takes the binned spread, or None."""
-    cells = prod(shape)
-    if points < _BINNED_POINTS or cells > 48 * points:
+    if points < _BINNED_POINTS or dtype not in _BINNED:
         return None
-    return max(12., 16. * (64000 + cells / 50) / points)
+    base, more, even, least, widest, most = _BINNED[dtype]
+    cells = prod(shape)
+    if cells > min(widest * points, most):
+        return None
+    return max(least, even * (base + more * min(cells / 64 ** 3, 1.) + cells / 50) / points)
 
 
 def _binned_bytes(grid, stencil, points, phi):
