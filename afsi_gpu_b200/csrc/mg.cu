@@ -26,9 +26,10 @@
 // changes in how it is executed, none in what is computed:
 //  * the mean-zero gauge (p -= mean after each smoothing block, rhs -= mean
 //    after restriction) is carried as a pending shift: the kernel that writes
-//    a field leaves one partial sum per block, and the next kernel that reads
-//    the field adds the partials in a fixed order (pending_mean) and subtracts
-//    sum/n on load, so no separate mean or subtract launches exist;
+//    a field leaves one partial sum per block (launches of many blocks: the
+//    finished sum), and the next kernel that reads the field adds the partials
+//    in a fixed order (pending_mean) and subtracts sum/n on load, so no separate
+//    mean or subtract launches exist;
 //  * zeroing the coarse iterate is folded into the first sweep (p_in = 0);
 //  * every level with at most kCoarseCells cells, the dense coarsest solve
 //    included, runs inside one thread block in shared memory.
@@ -51,7 +52,7 @@ namespace afsi {
 // diagonal; fast: the update p + (rhs - A p)(omega/diag) with omega/diag from a
 // 64-entry boundary-class table each block builds before waiting on its
 // predecessor (the single-CTA coarse levels use the same update).
-template <int BC, bool Exact, class T>
+template <int BC, bool Exact, class T, bool Wide>
 __global__ void __launch_bounds__(kThreads) sweep_kernel(const T* __restrict__ p, T* __restrict__ rhs, T* __restrict__ out,
                                                          Lv<T> L, Pending p_sum, Pending rhs_sum, Site emit,
                                                          int fix_rhs, int do_emit) {
@@ -63,8 +64,8 @@ __global__ void __launch_bounds__(kThreads) sweep_kernel(const T* __restrict__ p
     }
     pdl_enter();
     double local = 0.0;
-    const T m = T(pending_mean(p_sum, L.n));
-    const T mr = T(pending_mean(rhs_sum, L.n));
+    const T m = T(pending_mean<Wide>(p_sum, L.n));
+    const T mr = T(pending_mean<Wide>(rhs_sum, L.n));
     for_my_cells<BC>(L, [&](int x, int y, int z) {
         const int64_t i = index_of(x, y, z, L);
         T r = rhs[i];
@@ -93,7 +94,7 @@ __global__ void __launch_bounds__(kThreads) sweep_kernel(const T* __restrict__ p
         out[i] = v;
         local += double(v);
     });
-    if (do_emit) site_put(emit, local);
+    if (do_emit) site_leave<Wide>(emit, local);
 }
 
 // Two z-adjacent values.
@@ -171,7 +172,7 @@ __device__ __forceinline__ void pair_neg_lap(const ZPair<T>& c, const ZPair<T>& 
 // subtracts the rhs mean and writes it back.  Per cell the same operations in
 // the same order as sweep_kernel's fast form, so out is bitwise equal; the
 // emitted sum is added per block in this kernel's cell order.
-template <int BC, class T>
+template <int BC, class T, bool Wide>
 __global__ void __launch_bounds__(kThreads, 4) sweep_columns_kernel(const T* __restrict__ p, T* __restrict__ rhs,
                                                                     T* __restrict__ out, Lv<T> L, Pending rhs_sum,
                                                                     Site emit, int planes, int fix_rhs, int do_emit) {
@@ -186,7 +187,7 @@ __global__ void __launch_bounds__(kThreads, 4) sweep_columns_kernel(const T* __r
     const int x0 = int(blockIdx.z) * planes, x1 = min(x0 + planes, L.nx);
     pdl_enter();
     double local = 0.0;
-    const T mr = fix_rhs ? T(pending_mean(rhs_sum, L.n)) : T(0);
+    const T mr = fix_rhs ? T(pending_mean<Wide>(rhs_sum, L.n)) : T(0);
     if (z < L.nz && y < L.ny && x0 < x1) {
         const int64_t sx = int64_t(L.ny) * L.nz, sy = L.nz;
         int64_t i = (int64_t(x0) * L.ny + y) * L.nz + z;
@@ -239,14 +240,14 @@ __global__ void __launch_bounds__(kThreads, 4) sweep_columns_kernel(const T* __r
             c = after;
         }
     }
-    if (do_emit) site_put(emit, local);
+    if (do_emit) site_leave<Wide>(emit, local);
 }
 
 // residual_restrict_kernel's fast form for 3D levels (Neumann or Dirichlet)
 // with the fine z pairs of each coarse cell read as 16-byte vectors, each once
 // (the four pairs are each other's x and y neighbours): the eight children
 // summed in the same order (x, y, then z), so coarse is bitwise equal.
-template <int BC, class T>
+template <int BC, class T, bool Wide>
 __global__ void __launch_bounds__(kThreads) residual_restrict_zpair_kernel(const T* __restrict__ p,
                                                                           const T* __restrict__ rhs,
                                                                           T* __restrict__ coarse, Lv<T> L, Lv<T> C,
@@ -254,7 +255,7 @@ __global__ void __launch_bounds__(kThreads) residual_restrict_zpair_kernel(const
     using V = ZPair<T>;
     pdl_enter();
     double local = 0.0;
-    const T m = T(pending_mean(p_sum, L.n));
+    const T m = T(pending_mean<Wide>(p_sum, L.n));
     const int64_t sx = int64_t(L.ny) * L.nz, sy = L.nz;
     for_my_cells<BC>(C, [&](int cx, int cy, int cz) {
         const int64_t i = index_of(2 * cx, 2 * cy, 2 * cz, L);
@@ -296,32 +297,32 @@ __global__ void __launch_bounds__(kThreads) residual_restrict_zpair_kernel(const
         coarse[index_of(cx, cy, cz, C)] = v;
         local += double(v);
     });
-    if (do_emit) site_put(emit, local);
+    if (do_emit) site_leave<Wide>(emit, local);
 }
 
 // coarse[c] = mean of children of (rhs - A p), p shifted by m_p.  Launched
 // over the coarse lattice C.
-template <int BC, bool Exact, class T>
+template <int BC, bool Exact, class T, bool Wide>
 __global__ void __launch_bounds__(kThreads) residual_restrict_kernel(const T* __restrict__ p, const T* __restrict__ rhs,
                                                                      T* __restrict__ coarse, Lv<T> L, Lv<T> C,
                                                                      Pending p_sum, Site emit, int do_emit) {
     pdl_enter();
     double local = 0.0;
-    const T m = T(pending_mean(p_sum, L.n));
+    const T m = T(pending_mean<Wide>(p_sum, L.n));
     for_my_cells<BC>(C, [&](int cx, int cy, int cz) {
         const T v = restrict_residual_at<BC, Exact>(p, rhs, cx, cy, cz, L, m);
         coarse[index_of(cx, cy, cz, C)] = v;
         local += double(v);
     });
-    if (do_emit) site_put(emit, local);
+    if (do_emit) site_leave<Wide>(emit, local);
 }
 
 // dst = (src - m_src) + P(corr - m_corr); src may alias dst (own cell only).
-template <int BC, class T>
+template <int BC, class T, bool Wide>
 __global__ void __launch_bounds__(kThreads) prolong_kernel(const T* src, const T* __restrict__ corr, T* dst, Lv<T> L,
                                                            Lv<T> C, Pending src_sum, Pending corr_sum) {
     pdl_enter();
-    const T ms = T(pending_mean(src_sum, L.n)), mc = T(pending_mean(corr_sum, C.n));
+    const T ms = T(pending_mean<Wide>(src_sum, L.n)), mc = T(pending_mean<Wide>(corr_sum, C.n));
     for_my_cells<BC>(L, [&](int x, int y, int z) {
         const int64_t i = index_of(x, y, z, L);
         dst[i] = (src[i] - ms) + prolong_at<BC>(corr, x, y, z, C, mc);
@@ -333,12 +334,12 @@ __global__ void __launch_bounds__(kThreads) prolong_kernel(const T* src, const T
 // z and y interpolations they share serve eight cells (64 loads in
 // prolong_kernel).  Fine values are read and written as z pairs.  The same
 // interpolations in the same order per cell (z, then y, then x): bitwise equal.
-template <int BC, class T>
+template <int BC, class T, bool Wide>
 __global__ void __launch_bounds__(kThreads) prolong_octet_kernel(const T* src, const T* __restrict__ corr, T* dst,
                                                                  Lv<T> L, Lv<T> C, Pending src_sum, Pending corr_sum) {
     using V = ZPair<T>;
     pdl_enter();
-    const T ms = T(pending_mean(src_sum, L.n)), mc = T(pending_mean(corr_sum, C.n));
+    const T ms = T(pending_mean<Wide>(src_sum, L.n)), mc = T(pending_mean<Wide>(corr_sum, C.n));
     const bool odd = BC == AFSI_BC_DIRICHLET;  // ghosts are negated edge values (odd extension)
     const T near_ = T(.75), far_ = T(.25);
     for_my_cells<BC>(C, [&](int cx, int cy, int cz) {
@@ -663,8 +664,9 @@ Geometry launch_for(const Lv<T>& L, int bc) {
     g.block = dim3(bx, by, 1);
     const int gx = (fast + bx - 1) / bx, gy = (mid + by - 1) / by;
     // cap the blocks at 16 per SM of a B200 (x slabs beyond are strided inside
-    // the kernel), which bounds the arrivals at a reducing launch's completion
-    // counter; up to 64^3 every thread owns one cell
+    // the kernel), which bounds the partials that a consumer's blocks add or a
+    // last block completes; up to 64^3 every thread owns one cell.  A 2D grid and a
+    // y-z plane of its own are not capped (kPendingMost)
     const int cap = std::max(1, 2368 / std::max(1, gx * gy));
     g.grid = dim3(gx, gy, std::min(slow, cap));
     g.blocks = int64_t(g.grid.x) * g.grid.y * g.grid.z;
@@ -992,16 +994,20 @@ struct Runner {
         if (zpairs(l)) {
             int planes = 1;
             const Geometry g = launch_for_columns(L, &planes);
-            rc = launch_pdl("mg sweep", sweep_columns_kernel<BC, T>, g.grid, g.block, 0, stream, src, R(l), dst, L, rhs_sum,
-                            st.s[l][k], planes, rhs_sum.part ? 1 : 0, emit ? 1 : 0);
             blocks = g.blocks;
+            const auto kernel =
+                wide_launch(blocks) ? sweep_columns_kernel<BC, T, true> : sweep_columns_kernel<BC, T, false>;
+            rc = launch_pdl("mg sweep", kernel, g.grid, g.block, 0, stream, src, R(l), dst, L, rhs_sum,
+                            st.s[l][k], planes, rhs_sum.part ? 1 : 0, emit ? 1 : 0);
         } else {
             const Geometry g = launch_for(L, BC);
-            rc = launch_pdl("mg sweep", sweep_kernel<BC, false, T>, g.grid, g.block, 0, stream, src, R(l), dst, L, none,
-                            rhs_sum, st.s[l][k], rhs_sum.part ? 1 : 0, emit ? 1 : 0);
             blocks = g.blocks;
+            const auto kernel =
+                wide_launch(blocks) ? sweep_kernel<BC, false, T, true> : sweep_kernel<BC, false, T, false>;
+            rc = launch_pdl("mg sweep", kernel, g.grid, g.block, 0, stream, src, R(l), dst, L, none,
+                            rhs_sum, st.s[l][k], rhs_sum.part ? 1 : 0, emit ? 1 : 0);
         }
-        if (emit) *pending = Pending{st.s[l][k].partial, int(blocks)};
+        if (emit) *pending = pending_at(st.s[l][k], blocks);
         return rc;
     }
 
@@ -1025,29 +1031,31 @@ struct Runner {
         }
         const Lv<T>& C = lv[l + 1];
         const Geometry gc = launch_for(C, BC);
-        if (zpairs(l))
-            rc = launch_pdl("mg residual_restrict", residual_restrict_zpair_kernel<BC, T>, gc.grid, gc.block, 0, stream,
-                            static_cast<const T*>(cur), static_cast<const T*>(R(l)), R(l + 1), L, C, down_sum,
-                            st.s[l + 1][2], singular ? 1 : 0);
-        else
-            rc = launch_pdl("mg residual_restrict", residual_restrict_kernel<BC, false, T>, gc.grid, gc.block, 0, stream,
-                            static_cast<const T*>(cur), static_cast<const T*>(R(l)), R(l + 1), L, C, down_sum,
-                            st.s[l + 1][2], singular ? 1 : 0);
+        const bool wide = wide_launch(gc.blocks);
+        const auto pairs =
+            wide ? residual_restrict_zpair_kernel<BC, T, true> : residual_restrict_zpair_kernel<BC, T, false>;
+        const auto cells =
+            wide ? residual_restrict_kernel<BC, false, T, true> : residual_restrict_kernel<BC, false, T, false>;
+        rc = launch_pdl("mg residual_restrict", zpairs(l) ? pairs : cells, gc.grid, gc.block, 0, stream,
+                        static_cast<const T*>(cur), static_cast<const T*>(R(l)), R(l + 1), L, C, down_sum,
+                        st.s[l + 1][2], singular ? 1 : 0);
         if (rc) return rc;
         T* corr;
         Pending corr_sum;
-        const Pending coarse_rhs = singular ? Pending{st.s[l + 1][2].partial, int(gc.blocks)} : none;
+        const Pending coarse_rhs = singular ? pending_at(st.s[l + 1][2], gc.blocks) : none;
         if ((rc = level(l + 1, coarse_rhs, &corr, &corr_sum))) return rc;
         // the finest level of a singular operator prolongs into the buffer the
         // pre-smoothing left free, so its post-smoothing ends in Q(0) and the
         // finalize (and the fused check of the solve loop) never shifts in place
         T* pdst = (l == 0 && singular && cur == P(l)) ? Q(l) : P(l);
         if (zpairs(l)) {
-            rc = launch_pdl("mg prolong_add", prolong_octet_kernel<BC, T>, gc.grid, gc.block, 0, stream,
+            const auto octets = wide ? prolong_octet_kernel<BC, T, true> : prolong_octet_kernel<BC, T, false>;
+            rc = launch_pdl("mg prolong_add", octets, gc.grid, gc.block, 0, stream,
                             static_cast<const T*>(cur), static_cast<const T*>(corr), pdst, L, C, down_sum, corr_sum);
         } else {
             const Geometry g = launch_for(L, BC);
-            rc = launch_pdl("mg prolong_add", prolong_kernel<BC, T>, g.grid, g.block, 0, stream,
+            const auto kernel = wide_launch(g.blocks) ? prolong_kernel<BC, T, true> : prolong_kernel<BC, T, false>;
+            rc = launch_pdl("mg prolong_add", kernel, g.grid, g.block, 0, stream,
                             static_cast<const T*>(cur), static_cast<const T*>(corr), pdst, L, C, down_sum, corr_sum);
         }
         if (rc) return rc;
@@ -1251,14 +1259,16 @@ struct RbRunner {
                               static_cast<const TC*>(plan->coarse_inverse), int(lv[l].n));
         if ((rc = smooth(l))) return rc;
         const Geometry gc = launch_for(lv[l + 1], BC);
-        rc = launch_pdl("mg residual restrict", residual_restrict_kernel<BC, true, T>, gc.grid, gc.block, 0, stream,
+        const auto restrict_residual = wide_launch(gc.blocks) ? residual_restrict_kernel<BC, true, T, true>
+                                                              : residual_restrict_kernel<BC, true, T, false>;
+        rc = launch_pdl("mg residual restrict", restrict_residual, gc.grid, gc.block, 0, stream,
                         static_cast<const T*>(P(l)), static_cast<const T*>(R(l)), R(l + 1), lv[l], lv[l + 1],
-                        Pending{nullptr, 0}, st.s[l + 1][2], int(singular));
+                        Pending{nullptr, 0}, st.s[l + 1][2], singular ? 1 : 0);
         if (rc) return rc;
         if (singular) {
             rc = launch_pdl("mg mean shift", shift_kernel<T>, dim3(flat_grid(lv[l + 1].n)), dim3(kThreads), 0, stream,
                             static_cast<const T*>(R(l + 1)), R(l + 1), lv[l + 1].n,
-                            Pending{st.s[l + 1][2].partial, int(gc.blocks)});
+                            pending_at(st.s[l + 1][2], gc.blocks));
             if (rc) return rc;
         }
         if (l + 1 < last && l + 1 != first_coarse) {
@@ -1267,7 +1277,7 @@ struct RbRunner {
         }
         if ((rc = level(l + 1))) return rc;
         const Geometry g = launch_for(lv[l], BC);
-        rc = launch_pdl("mg prolong add", prolong_kernel<BC, T>, g.grid, g.block, 0, stream,
+        rc = launch_pdl("mg prolong add", prolong_kernel<BC, T, false>, g.grid, g.block, 0, stream,
                         static_cast<const T*>(P(l)), static_cast<const T*>(P(l + 1)), P(l), lv[l], lv[l + 1],
                         Pending{nullptr, 0}, Pending{nullptr, 0});
         if (rc) return rc;
@@ -1632,7 +1642,7 @@ extern "C" int32_t afsi_b200_mg_smooth(const void* p, const void* rhs, void* out
             Lv<T> L = make_level<T>(shape, h2, inv_h2, dim);
             const Geometry g = launch_for(L, BC);
             Site none{nullptr, nullptr, nullptr};
-            sweep_kernel<BC, true, T><<<g.grid, g.block, 0, stream>>>(
+            sweep_kernel<BC, true, T, false><<<g.grid, g.block, 0, stream>>>(
                 static_cast<const T*>(p), const_cast<T*>(static_cast<const T*>(rhs)), static_cast<T*>(out), L,
                 Pending{nullptr, 0}, Pending{nullptr, 0}, none, 0, 0);
         });
@@ -1694,7 +1704,7 @@ extern "C" int32_t afsi_b200_mg_residual_restrict(const void* p, const void* rhs
             Lv<T> C = coarser(L);
             const Geometry g = launch_for(C, BC);
             Site none{nullptr, nullptr, nullptr};
-            residual_restrict_kernel<BC, true, T><<<g.grid, g.block, 0, stream>>>(
+            residual_restrict_kernel<BC, true, T, false><<<g.grid, g.block, 0, stream>>>(
                 static_cast<const T*>(p), static_cast<const T*>(rhs), static_cast<T*>(coarse), L, C, Pending{nullptr, 0},
                 none, 0);
         });
@@ -1714,7 +1724,7 @@ extern "C" int32_t afsi_b200_mg_prolong_add(const void* coarse, void* fine, cons
             Lv<T> L = make_level<T>(shape, one, one, dim);
             Lv<T> C = coarser(L);
             const Geometry g = launch_for(L, BC);
-            prolong_kernel<BC, T><<<g.grid, g.block, 0, stream>>>(static_cast<const T*>(fine),
+            prolong_kernel<BC, T, false><<<g.grid, g.block, 0, stream>>>(static_cast<const T*>(fine),
                                                                   static_cast<const T*>(coarse), static_cast<T*>(fine),
                                                                   L, C, Pending{nullptr, 0}, Pending{nullptr, 0});
         });

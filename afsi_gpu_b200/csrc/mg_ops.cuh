@@ -279,11 +279,13 @@ struct Pending {
 
 // Mean of a pending sum over n cells, the same bits in every thread of every
 // block whatever the block's size: warp 0 adds partials l, l + 32, ... per lane
-// and then a fixed tree.  Summing a few hundred partials in each consumer
-// block costs one L2 round trip; completing the sum in the producer cost a
-// fence, a counter and a last block at the end of every emitting launch.
+// and then a fixed tree, four loads in flight: 592 partials (a wave of sweeps)
+// are five L2 round trips.
+// Wide: a launch of many blocks, whose sums are finished ones (see kPendingMost).
+template <bool Wide = false>
 __device__ __forceinline__ double pending_mean(Pending s, int64_t n) {
     if (!s.part) return 0.0;
+    if (Wide && s.count == 1) return __ldcg(s.part) / double(n);
     __shared__ double mean;
     const unsigned t = thread_linear();
     if (t < 32) {
@@ -305,6 +307,23 @@ __device__ __forceinline__ void site_put(const Site& s, double v) {
     __shared__ double warp_sums[32];
     v = block_sum2(v, warp_sums);
     if (thread_linear() == 0) s.partial[block_linear()] = v;
+}
+
+// Blocks up to which a producer leaves its partials to the consumers.  Every
+// block of a consumer adds all of them, so the work is their product, and the
+// grids of 2D levels are not capped (launch_for): beyond, the producer's last
+// block completes the sum after a fence and a counter.  A cycle of a periodic
+// channel, one B200, partials always / as here / last block always: 512 x 512 (1024
+// blocks) 139 / 137 / 148 us, 1024 x 512 177 / 171 / 180, 1024 x 1024 286 / 243 / 242,
+// 2048 x 2048 1226 / 623 / 618, 4096 x 4096 11520 / 2239 / 2129; 128^3 207 / 205 / 233
+// (restriction: 1024 blocks).
+constexpr int kPendingMost = 1200;
+
+inline bool wide_launch(int64_t blocks) { return blocks > kPendingMost; }
+
+// What a producer of so many blocks leaves at its site.
+inline Pending pending_at(const Site& s, int64_t blocks) {
+    return wide_launch(blocks) ? Pending{s.result, 1} : Pending{s.partial, int(blocks)};
 }
 
 // Block partial + last-block completion for a grid reduction of `v`.
@@ -330,6 +349,16 @@ __device__ __forceinline__ void site_finish(const Site& s, double v, double* sqr
         else *s.result = acc;
         *s.counter = 0u;
     }
+}
+
+// This block's share of a field's sum, left as the launch's width says (a variant
+// of the kernel each: both in one cost every sweep of the small grids 0.1 us).
+template <bool Wide>
+__device__ __forceinline__ void site_leave(const Site& s, double v) {
+    if constexpr (Wide)
+        site_finish(s, v);
+    else
+        site_put(s, v);
 }
 
 // site_finish, then tail(result) in thread 0 of the last block, after the

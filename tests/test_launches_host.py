@@ -19,7 +19,7 @@ spec.loader.exec_module(L)
 HOOK = ctypes.CFUNCTYPE(None, ctypes.c_char_p, ctypes.c_int, ctypes.c_uint, ctypes.c_size_t,
                         ctypes.POINTER(ctypes.c_void_p))
 log = []
-hook = HOOK(lambda name, device, blocks, smem, args: log.append((name.decode(), device, blocks, smem, look(name, args))))
+hook = HOOK(lambda name, device, blocks, smem, args: log.append((name.decode(), device, blocks, smem, look(name.decode(), args))))
 look = lambda name, args: None
 L.load()
 fake.fake_hook(hook)
@@ -93,3 +93,64 @@ print(len(seen[0]), max(smem for _, _, smem in seen[0]))
 ''')
     launches, largest = map(int, out.split())
     assert launches > 100 and largest > 48 * 1024
+
+
+def test_no_consumer_adds_thousands_of_partials(run):
+    """Pending means: every block of a consumer adds all partials of its producer,
+    so grids of thousands of blocks must leave one finished sum instead; and what a
+    consumer reads is what the producer of that field left."""
+    run('''
+MOST = 1200  # kPendingMost
+
+class Pending(ctypes.Structure):
+    _fields_ = [('part', ctypes.c_void_p), ('count', ctypes.c_int)]
+
+class Site(ctypes.Structure):
+    _fields_ = [('partial', ctypes.c_void_p), ('counter', ctypes.c_void_p), ('result', ctypes.c_void_p)]
+
+READS = {'sweep_kernel': (4, 5), 'sweep_columns_kernel': (4,), 'residual_restrict_zpair_kernel': (5,),
+         'residual_restrict_kernel': (5,), 'prolong_kernel': (5, 6), 'prolong_octet_kernel': (5, 6),
+         'shift_kernel': (3,), 'coarse_kernel': (1,), 'cluster_kernel': (1,)}
+LEAVES = {'sweep_kernel': (6, 8), 'sweep_columns_kernel': (5, 8), 'residual_restrict_zpair_kernel': (6, 7),
+          'residual_restrict_kernel': (6, 7), 'level_sum_kernel': (2, None)}  # site, flag (none: always)
+of = lambda args, i, kind: ctypes.cast(args[i], ctypes.POINTER(kind))[0]
+
+def look(name, args):
+    kernel = [k for k in sorted({**READS, **LEAVES}, key=len, reverse=True) if f'{len(k)}{k}I' in name]
+    if not kernel:
+        return None
+    k = kernel[0]
+    reads = [(p.part, p.count) for p in (of(args, i, Pending) for i in READS.get(k, ())) if p.part]
+    site, mode = None, 0
+    if k in LEAVES:
+        at, i = LEAVES[k]
+        site = of(args, at, Site)
+        if i is None or of(args, i, ctypes.c_int):
+            mode = 2 if i is None or 'Lb1EE' in name else 1  # the last template argument: finished by the producer
+        site = site.partial, site.result
+    return k, reads, site, mode
+
+for shape, bc, levels in (((256, 128), L.BC_PERIODIC, 5), ((1024, 512), L.BC_PERIODIC, 7), ((2048, 512), L.BC_PERIODIC, 7),
+                          ((4096, 4096), L.BC_PERIODIC, 9), ((64, 64, 64), L.BC_NEUMANN, 5),
+                          ((256, 256, 256), L.BC_NEUMANN, 6), ((64, 512, 512), L.BC_NEUMANN, 6),
+                          ((128, 1024, 512), L.BC_NEUMANN, 7)):
+    for smoother in (0, 1):
+        for dt in (L.F64, L.F32):
+            p = plan(shape, bc, levels, dt)
+            p.smoother = smoother
+            log.clear()
+            L.call('afsi_b200_mg_vcycles', ctypes.byref(p), 2, None)
+            left, read = {}, 0
+            for name, device, blocks, smem, seen in log:
+                if seen is None:
+                    continue
+                kernel, reads, site, mode = seen
+                for part, count in reads:
+                    assert count <= MOST, (shape, kernel, count)
+                    assert left[part] == count, (shape, kernel)
+                    read += 1
+                if mode:
+                    left.pop(site[0], None), left.pop(site[1], None)
+                    left[site[0 if mode == 1 else 1]] = blocks if mode == 1 else 1
+            assert read, shape
+''')
