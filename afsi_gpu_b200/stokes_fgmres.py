@@ -95,8 +95,9 @@ class _Arnoldi:
     def step(self, j, w):
         """w against V[:j+1]; V[j+1] set; the Hessenberg column and ||w|| (host)."""
         w = w.contiguous()
-        call('afsi_b200_krylov_step', ptr(self.V), self.n, j + 1, ptr(w), ptr(self.work), ptr(self.column),
-             ptr(self.scratch), self.scratch.numel(), dtype_code(w.dtype), stream(w.device))
+        with torch.cuda.device(self.V.device):  # the vectors' device need not be the current one
+            call('afsi_b200_krylov_step', ptr(self.V), self.n, j + 1, ptr(w), ptr(self.work), ptr(self.column),
+                 ptr(self.scratch), self.scratch.numel(), dtype_code(w.dtype), stream(w.device))
         return self.column[:j + 3].tolist()
 
 
