@@ -149,7 +149,10 @@ __global__ void __launch_bounds__(kDetWarps * 32) det_tile_kernel(const T* __res
                               rz = det_row(g.total, p, c, 2);
                 const int lx = int(base[rx] - t0[0]) + li, ly = int(base[ry] - t0[1]) + lj,
                           lz = int(base[rz] - t0[2]) + kz;
-                off[u] = (lx * kHalo + ly) * kHalo + lz;
+                // outside: the rows were written anew since the plan was made (left out, whole or in part)
+                const bool in = unsigned(lx) < unsigned(kHalo) && unsigned(ly) < unsigned(kHalo) &&
+                                unsigned(lz) < unsigned(kHalo - 1);
+                off[u] = in ? (lx * kHalo + ly) * kHalo + lz : -1;
                 w[u] = phi[rx * 4 + li] * phi[ry * 4 + lj];
                 z0[u] = phi[rz * 4 + kz];
                 z1[u] = phi[rz * 4 + kz + 1];

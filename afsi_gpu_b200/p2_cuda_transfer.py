@@ -29,7 +29,7 @@ word by the transfers and raised by ``confirm``.  ``P1Transfer`` is the
 matrix-free P1 element transfer (``mac/adaptive_cell.py:22-83``) on the same
 kernels with four-node cells.
 """
-from dataclasses import dataclass
+from dataclasses import dataclass, field
 import torch
 from . import _lib
 from ._lib import call, ptr, stream, dtype_code
@@ -61,6 +61,8 @@ class SharedAdaptiveStencil:
     base: torch.Tensor   # (2,T,3) int64: lattice 0 = faces, 1 = centres
     phi: torch.Tensor    # (2,T,3,4)
     rule: InteractionRule
+    # sorted rows of the deterministic spread (P2Transfer.det_plan): they live and end with these tables
+    plans: dict = field(default_factory=dict, init=False, repr=False, compare=False)
     layout = 'shared'
 
     @property
@@ -242,11 +244,13 @@ class P2Transfer:
         return spread(self, coefficient, stencil)
 
     def det_plan(self, stencil):
-        """Tile-sorted rows of `stencil` for the deterministic spread (built once per stencil)."""
-        key = (stencil.base.data_ptr(), stencil.base.shape[1], stencil.phi.dtype)
-        if getattr(self, '_det', None) is not None and self._det[0] == key:
-            return self._det[1]
+        """Tile-sorted rows of `stencil` for the deterministic spread, built once per
+        stencil and kept by it: the next step's tables may lie at the same address."""
         g = self.grid
+        version = 0 if stencil.base.is_inference() else stencil.base._version
+        key = (tuple(g.shape), stencil.phi.dtype, version)
+        if key in stencil.plans:
+            return stencil.plans[key]
         total = stencil.base.shape[1]
         code = dtype_code(stencil.phi.dtype)
         n = _lib.load().afsi_b200_det_plan_bytes(total, *g.shape, code)
@@ -261,7 +265,8 @@ class P2Transfer:
         if flags:
             word.zero_()
             raise RuntimeError('P2 stencil support outside the MAC face arrays')
-        self._det = (key, plan)
+        stencil.plans.clear()
+        stencil.plans[key] = plan
         return plan
 
     def assemble_velocity(self, velocity, stencil):
