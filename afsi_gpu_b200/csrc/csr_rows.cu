@@ -18,8 +18,11 @@
 //              adds each sum, FP32 adds point by point;
 //              the touched entries leave the box in ascending face order, which
 //              is the CSR column order: B needs no sort.  An entry exists when
-//              some contribution is nonzero (untouched entries hold -0, which no
-//              sum of nonzero terms gives);
+//              something nonzero was added to it (untouched entries hold -0, which
+//              no sum of nonzero terms gives): in FP32 a point's product, in FP64
+//              the sum of one origin's points among the 32 staged, in the hash
+//              form a cell's sum.  The three differ where contributions of either
+//              sign cancel exactly, and then in explicit zeros;
 //   finish     the padded rows packed to CSR, and the transpose by a stable
 //              radix sort on the face index alone (32-bit keys and positions).
 //
