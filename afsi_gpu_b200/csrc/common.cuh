@@ -6,6 +6,7 @@
 // that want a fused multiply-add say so with fma().
 #pragma once
 #include <atomic>
+#include <cmath>
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <math.h>
@@ -123,12 +124,6 @@ __device__ __forceinline__ double sum_partials(const double* partial, int count,
     return block_sum(v, shared);
 }
 
-// Programmatic dependent launch (sm_90+): let the next kernel in the stream
-// begin launching now, then wait until every kernel this one depends on has
-// completed and its writes are visible.  The next kernel is launched only
-// after every block of this one has started, so waiting blocks never hold back
-// a kernel they depend on.  Both are no-ops for a launch without the
-// programmatic-serialization attribute.
 // 1/v when v is a positive normal power of two whose reciprocal is normal
 // (then x * (1/v) rounds exactly as x / v), else 0.
 template <class T>
@@ -144,11 +139,25 @@ __device__ __forceinline__ T exact_reciprocal(T v) {
     }
 }
 
+// The same on the host.
+template <class T>
+T exact_inverse(T v) {
+    int ex = 0;
+    const T inv = T(1) / v;
+    return std::isnormal(v) && std::isnormal(inv) && std::frexp(double(v), &ex) == 0.5 ? inv : T(0);
+}
+
 // The four faces of a support that starts at b lie inside [0, n).  Any table
 // entry: points without a support check bin to the ends of the 64-bit range,
 // where b + 3 wraps.
 __host__ __device__ __forceinline__ bool support_inside(int64_t b, int64_t n) { return b >= 0 && b <= n - 4; }
 
+// Programmatic dependent launch (sm_90+): let the next kernel in the stream
+// begin launching now, then wait until every kernel this one depends on has
+// completed and its writes are visible.  The next kernel is launched only
+// after every block of this one has started, so waiting blocks never hold back
+// a kernel they depend on.  Both are no-ops for a launch without the
+// programmatic-serialization attribute.
 __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_enter() {

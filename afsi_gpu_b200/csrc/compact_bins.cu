@@ -173,92 +173,59 @@ __global__ void __launch_bounds__(kBinWarps * 32, 5) bin_spread_kernel(
     T* __restrict__ u0, T* __restrict__ u1, T* __restrict__ u2, int32_t* status) {
     extern __shared__ __align__(16) unsigned char bin_smem[];
     BinStage<T>& s = reinterpret_cast<BinStage<T>*>(bin_smem)[threadIdx.x >> 5];
-    constexpr int J = kBinPoints / 32;
+    static_assert(kBinPoints == 32, "a point per lane");
     const int lane = threadIdx.x & 31;
     const int64_t chunk = int64_t(blockIdx.x) * kBinWarps + (threadIdx.x >> 5), q0 = chunk * kBinPoints;
     if (q0 >= points) return;  // whole warp
     const int n = int(points - q0 < kBinPoints ? points - q0 : kBinPoints);
     if (lane < 12) s.w[kBinPoints * 12 + lane] = T(0);
     if (lane == 0) s.f[kBinPoints] = T(0);
-#pragma unroll
-    for (int j = 0; j < J; ++j) s.id[lane + 32 * j] = lane + 32 * j < n ? order[q0 + lane + 32 * j] : 0;
+    const bool mine = lane < n;
+    s.id[lane] = mine ? order[q0 + lane] : 0;
     __syncwarp();
     bin_fetch_rows(s, phi, points, 0, n);
-    T force_of[J][3];
+    T force_of[3];
 #pragma unroll
-    for (int j = 0; j < J; ++j)
+    for (int c = 0; c < 3; ++c) force_of[c] = mine ? force[int64_t(s.id[lane]) * 3 + c] : T(0);
 #pragma unroll
-        for (int c = 0; c < 3; ++c)
-            force_of[j][c] = lane + 32 * j < n ? force[int64_t(s.id[lane + 32 * j]) * 3 + c] : T(0);
-#pragma unroll
-    for (int i = 0; i < 9 * J; ++i) {  // 3 components, 3 J rounds of 32 coordinates
-        const int c = i / (3 * J), t = lane + 32 * (i - c * 3 * J), q = t / 3;
+    for (int i = 0; i < 9; ++i) {  // 3 components, 3 rounds of 32 coordinates
+        const int c = i / 3, t = lane + 32 * (i - c * 3), q = t / 3;
         const int64_t v = q < n ? base[(c * points + s.id[q]) * 3 + (t - 3 * q)] : -1;
         s.b[c][t] = v >= 0 && v < kBinOut ? uint16_t(v) : kBinOut;
     }
     __syncwarp();
-    unsigned tile[J];
-#pragma unroll
-    for (int j = 0; j < J; ++j) {
-        const uint16_t* b0 = s.b[0] + (lane + 32 * j) * 3;
-        const unsigned k = bin_key(b0[0], b0[1], b0[2], g);
-        tile[j] = k == g.none ? 0xfffffffeu : k >> 6;
-    }
+    const uint16_t* b0 = s.b[0] + lane * 3;
+    const unsigned cell = bin_key(b0[0], b0[1], b0[2], g), tile = cell == g.none ? 0xfffffffeu : cell >> 6;
 #pragma unroll 1
     for (int c = 0; c < 3; ++c) {
         T* field = c == 0 ? u0 : c == 1 ? u1 : u2;
         const int e0 = bin_extent(g, c, 0), e1 = bin_extent(g, c, 1), e2 = bin_extent(g, c, 2);
-        int b[J][3];
-        bool live[J];
+        int b[3];
 #pragma unroll
-        for (int j = 0; j < J; ++j) {
-            const int q = lane + 32 * j;
-#pragma unroll
-            for (int a = 0; a < 3; ++a) b[j][a] = s.b[c][q * 3 + a];
-            live[j] = q < n && b[j][0] + 3 < e0 && b[j][1] + 3 < e1 && b[j][2] + 3 < e2;
-            if (q < n && !live[j]) flag(status, AFSI_FLAG_INDEX);
-            const T fv = c == 0 ? force_of[j][0] : c == 1 ? force_of[j][1] : force_of[j][2];
-            if (q < n) s.f[q] = inv_volume != T(0) ? fv * inv_volume : fv / volume;
-        }
+        for (int a = 0; a < 3; ++a) b[a] = s.b[c][lane * 3 + a];
+        const bool live = mine && b[0] + 3 < e0 && b[1] + 3 < e1 && b[2] + 3 < e2;
+        if (mine && !live) flag(status, AFSI_FLAG_INDEX);
+        const T fv = c == 0 ? force_of[0] : c == 1 ? force_of[1] : force_of[2];
+        if (mine) s.f[lane] = inv_volume != T(0) ? fv * inv_volume : fv / volume;
         asm volatile("cp.async.wait_all;" ::: "memory");
         __syncwarp();
         // the whole warp at once when one box covers it, else tile by tile
-        bool left[J];
-#pragma unroll
-        for (int j = 0; j < J; ++j) left[j] = live[j];
-        bool whole = true, fetched = c == 2;  // the next component's rows
+        bool left = live, whole = true, fetched = c == 2;  // fetched: the next component's rows
         while (true) {
-            bool some = false;
-            unsigned now = 0;  // the tile of a point that is left
-#pragma unroll
-            for (int j = 0; j < J; ++j) {
-                const unsigned m = __ballot_sync(0xffffffffu, left[j]);
-                if (m) now = __shfl_sync(0xffffffffu, tile[j], __ffs(m) - 1);
-                some = some || m;
-            }
-            if (!some) {
+            const unsigned rest = __ballot_sync(0xffffffffu, left);
+            if (!rest) {
                 if (!fetched) bin_fetch_rows(s, phi, points, c + 1, n);  // no point of this component
                 break;
             }
-            bool take[J];
-            int mn[3] = {INT_MAX, INT_MAX, INT_MAX}, mx[3] = {INT_MIN, INT_MIN, INT_MIN};
-#pragma unroll
-            for (int j = 0; j < J; ++j) {
-                take[j] = left[j] && (whole || tile[j] == now);
-                if (take[j])
-#pragma unroll
-                    for (int a = 0; a < 3; ++a) {
-                        mn[a] = min(mn[a], b[j][a]);
-                        mx[a] = max(mx[a], b[j][a]);
-                    }
-            }
+            const unsigned now = __shfl_sync(0xffffffffu, tile, __ffs(rest) - 1);  // the tile of a point that is left
+            const bool take = left && (whole || tile == now);
+            int mn[3], mx[3];
 #pragma unroll
             for (int a = 0; a < 3; ++a) {
-                mn[a] = __reduce_min_sync(0xffffffffu, mn[a]);
-                mx[a] = __reduce_max_sync(0xffffffffu, mx[a]);
+                mn[a] = __reduce_min_sync(0xffffffffu, take ? b[a] : INT_MAX);
+                mx[a] = __reduce_max_sync(0xffffffffu, take ? b[a] : INT_MIN);
             }
-#pragma unroll
-            for (int j = 0; j < J; ++j) left[j] = left[j] && !take[j];
+            left = left && !take;
             const int ex = mx[0] - mn[0] + 4, ey = mx[1] - mn[1] + 4, ez = mx[2] - mn[2] + 4;
             int sx = 0, sy = 0;
             bool fits = ey <= 64 && ez <= 64;
@@ -268,36 +235,23 @@ __global__ void __launch_bounds__(kBinWarps * 32, 5) bin_spread_kernel(
             }
             if (whole && !fits) {
                 whole = false;
-#pragma unroll
-                for (int j = 0; j < J; ++j) left[j] = live[j];
+                left = live;
                 continue;
             }
-            bool mine = false;
-            int count = 0;
-#pragma unroll
-            for (int j = 0; j < J; ++j) {
-                mine = mine || left[j];
-                count += __popc(__ballot_sync(0xffffffffu, take[j]));
-            }
-            const bool fetch = !fetched && !__any_sync(0xffffffffu, mine);
+            const unsigned taken = __ballot_sync(0xffffffffu, take);
+            const int count = __popc(taken);
+            const bool fetch = !fetched && !__any_sync(0xffffffffu, left);
             fetched = fetched || fetch;
             if (fits && count >= kBinFew) {
                 const int size = ex * sx;
                 for (int t = lane; t < size; t += 32) s.box[t] = T(0);
-                int key[J], runs = 0;
-#pragma unroll
-                for (int j = 0; j < J; ++j) {
-                    key[j] = take[j] ? run_key(b[j][0] - mn[0], b[j][1] - mn[1], b[j][2] - mn[2]) : -1;
-                    const unsigned peers = __match_any_sync(0xffffffffu, key[j]);
-                    runs += __popc(__ballot_sync(0xffffffffu, take[j] && (peers & ((1u << lane) - 1u)) == 0u));
-                }
+                const int d0 = b[0] - mn[0], d1 = b[1] - mn[1], d2 = b[2] - mn[2];
+                int key = take ? run_key(d0, d1, d2) : -1;
+                const unsigned peers = __match_any_sync(0xffffffffu, key);
+                const int runs = __popc(__ballot_sync(0xffffffffu, take && (peers & ((1u << lane) - 1u)) == 0u));
                 const bool merge = count >= kBinMerge * runs;
-#pragma unroll
-                for (int j = 0; j < J; ++j) {
-                    const int k = key[j];
-                    if (!merge && take[j]) key[j] = (k & 1023) * sx + ((k >> 10) & 1023) * sy + (k >> 20);
-                    s.key[lane + 32 * j] = key[j];
-                }
+                if (!merge && take) key = d0 * sx + d1 * sy + d2;
+                s.key[lane] = key;
                 __syncwarp();
                 if (merge)
                     spread_element<T, kBinPoints>(s.box, s.key, s.f, s.w, s.w + 4, s.w + 8, n, sx, sy, s.perm, s.rs,
@@ -324,29 +278,23 @@ __global__ void __launch_bounds__(kBinWarps * 32, 5) bin_spread_kernel(
                 __syncwarp();
             } else {  // four lanes per point, lane k on z link k, as the plain form
                 __syncwarp();
-#pragma unroll
-                for (int j = 0; j < J; ++j) {
-                    unsigned todo = __ballot_sync(0xffffffffu, take[j]);
-                    while (todo) {
-                        // up to eight points at a time
-                        int src = 0;
-                        unsigned rest = todo;
-                        for (int k = 0; k < (lane >> 2) && rest; ++k) rest &= rest - 1;
-                        const bool has = rest != 0;
-                        src = has ? __ffs(rest) - 1 : 0;
-                        const int bx = __shfl_sync(0xffffffffu, b[j][0], src), by = __shfl_sync(0xffffffffu, b[j][1], src),
-                                  bz = __shfl_sync(0xffffffffu, b[j][2], src);
-                        if (has) {
-                            const T* w = s.w + (src + 32 * j) * 12;
-                            const int k = lane & 3;
-                            const T fz = s.f[src + 32 * j] * w[8 + k];
-                            T* dst = field + (int64_t(bx) * e1 + by) * e2 + bz + k;
-                            for (int i = 0; i < 4; ++i)
-                                for (int l = 0; l < 4; ++l)
-                                    atomicAdd(dst + (int64_t(i) * e1 + l) * e2, (w[i] * w[4 + l]) * fz);
-                        }
-                        for (int k = 0; k < 8 && todo; ++k) todo &= todo - 1;
+                for (unsigned todo = taken; todo;) {  // up to eight points at a time
+                    unsigned next = todo;
+                    for (int k = 0; k < (lane >> 2) && next; ++k) next &= next - 1;
+                    const bool has = next != 0;
+                    const int src = has ? __ffs(next) - 1 : 0;
+                    const int bx = __shfl_sync(0xffffffffu, b[0], src), by = __shfl_sync(0xffffffffu, b[1], src),
+                              bz = __shfl_sync(0xffffffffu, b[2], src);
+                    if (has) {
+                        const T* w = s.w + src * 12;
+                        const int k = lane & 3;
+                        const T fz = s.f[src] * w[8 + k];
+                        T* dst = field + (int64_t(bx) * e1 + by) * e2 + bz + k;
+                        for (int i = 0; i < 4; ++i)
+                            for (int l = 0; l < 4; ++l)
+                                atomicAdd(dst + (int64_t(i) * e1 + l) * e2, (w[i] * w[4 + l]) * fz);
                     }
+                    for (int k = 0; k < 8 && todo; ++k) todo &= todo - 1;
                 }
                 __syncwarp();
                 if (fetch) bin_fetch_rows(s, phi, points, c + 1, n);
@@ -420,13 +368,11 @@ extern "C" int32_t afsi_b200_compact_spread3_binned(const void* force, const int
     if (rc) return rc;
     AFSI_DISPATCH(dtype, {
         const T vol = T(volume);
-        int ex = 0;
-        const T inv = std::frexp(double(vol), &ex) == 0.5 && std::isnormal(T(1) / vol) ? T(1) / vol : T(0);
         const size_t smem = sizeof(BinStage<T>) * kBinWarps;
         if ((rc = allow_shared<bin_spread_kernel<T>>("compact_spread3_binned", smem))) return rc;
         const int64_t warps = (points + kBinPoints - 1) / kBinPoints;
         bin_spread_kernel<T><<<blocks_for(warps, kBinWarps), kBinWarps * 32, smem, stream>>>(
-            static_cast<const T*>(force), base, static_cast<const T*>(phi), points, order, g, vol, inv,
+            static_cast<const T*>(force), base, static_cast<const T*>(phi), points, order, g, vol, exact_inverse(vol),
             static_cast<T*>(u0), static_cast<T*>(u1), static_cast<T*>(u2), status);
     });
     return launched("compact_spread3_binned");

@@ -1196,13 +1196,8 @@ Geo<TP> make_geo(const double* origin, const double* spacing, const double* limi
         geo.origin[a] = TP(origin[a]);
         geo.spacing[a] = TP(spacing[a]);
         geo.limits[a] = TP(limits[a]);
-        int ex = 0;
-        const TP h = geo.spacing[a];
-        // a power of two: its reciprocal is exact and x * (1/h) rounds as x / h
-        const bool pow2 = std::isfinite(double(h)) && h > TP(0) && std::frexp(double(h), &ex) == 0.5 &&
-                          TP(1) / h == TP(std::ldexp(1.0, 1 - ex)) && std::isnormal(double(TP(1) / h));
-        geo.inv[a] = pow2 ? TP(1) / h : TP(0);
-        if (pow2) geo.pow2 |= 1 << a;
+        geo.inv[a] = exact_inverse(geo.spacing[a]);
+        if (geo.inv[a] != TP(0)) geo.pow2 |= 1 << a;
     }
     return geo;
 }
@@ -1269,13 +1264,11 @@ extern "C" int32_t afsi_b200_fe_fused_spread(int32_t nodes_per_cell, const void*
             const size_t multi = sizeof(MStage<TP, T, NPC>) * kMWarps;
             if ((rc = allow_shared<fused_spread_multi_kernel<TP, T, NPC>>("fused_spread_multi", multi))) return rc;
             const T vol = T(volume);
-            int ex = 0;
-            const bool pow2 = std::frexp(double(vol), &ex) == 0.5 && std::isnormal(T(1) / vol);
             fused_spread_multi_kernel<TP, T, NPC>
                 <<<fused_blocks((elements + G - 1) / G, kMWarps), kMWarps * 32, multi, s>>>(
                     static_cast<const TP*>(x), cells, static_cast<const TP*>(N_pos), static_cast<const T*>(N),
                     static_cast<const T*>(W), static_cast<const T*>(value), make_geo<TP>(origin, spacing, limits),
-                    static_cast<T*>(u0), static_cast<T*>(u1), static_cast<T*>(u2), g, G, vol, pow2 ? T(1) / vol : T(0),
+                    static_cast<T*>(u0), static_cast<T*>(u1), static_cast<T*>(u2), g, G, vol, exact_inverse(vol),
                     status);
             return launched("fused_spread_multi");
         }

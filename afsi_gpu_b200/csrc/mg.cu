@@ -680,10 +680,8 @@ Geometry launch_for(const Lv<T>& L, int bc) {
 template <class T>
 bool divides_exactly(const Lv<T>& L, int dim) {
     for (int a = 0; a < dim; ++a) {
-        int ex = 0;
-        if (!(std::isnormal(L.h2[a]) && std::frexp(double(L.h2[a]), &ex) == 0.5 && std::isnormal(L.ih2[a]) &&
-              L.ih2[a] == T(1) / L.h2[a]))
-            return false;
+        const T inv = exact_inverse(L.h2[a]);
+        if (inv == T(0) || L.ih2[a] != inv) return false;
     }
     return true;
 }

@@ -30,15 +30,8 @@ namespace afsi {
 constexpr int kCells = 256;  // cells (threads) per block, one partial per block
 
 struct Cells {
-    int64_t nx, ny, nz;  // pressure cells
+    int64_t nx, ny, nz;  // pressure cells; faces: (nx+1, ny, nz), (nx, ny+1, nz), (nx, ny, nz+1)
 };
-
-// Face array of component c: (nx+1, ny, nz), (nx, ny+1, nz), (nx, ny, nz+1).
-__device__ __forceinline__ void face_dims(const Cells& g, int c, int64_t* n) {
-    n[0] = g.nx + (c == 0);
-    n[1] = g.ny + (c == 1);
-    n[2] = g.nz + (c == 2);
-}
 
 template <class T>
 struct Faces {
@@ -364,13 +357,6 @@ dim3 march_grid(const Cells& g, int* chunks) {
     return dim3(unsigned(bx), unsigned(3 * *chunks));
 }
 
-// 1/v where v is a power of two whose inverse is normal, else 0.
-template <class T>
-T power_of_two_inverse(T v) {
-    int ex = 0;
-    return v > T(0) && std::isnormal(v) && std::frexp(double(v), &ex) == 0.5 && std::isnormal(T(1) / v) ? T(1) / v : T(0);
-}
-
 unsigned cell_blocks(const Cells& g) { return unsigned((g.nx * g.ny * g.nz + kCells - 1) / kCells); }
 
 }  // namespace
@@ -416,7 +402,7 @@ extern "C" int32_t afsi_b200_helmholtz_sweep(const void* const* u, const void* c
         const T h2[3] = {T(spacing_squared[0]), T(spacing_squared[1]), T(spacing_squared[2])};
         return launch_pdl("helmholtz sweep", helmholtz_sweep_kernel<T>, grid, dim3(256), 0, stream, cfaces<T>(u),
                           cfaces<T>(rhs), cfaces<T>(diag), faces<T>(out), static_cast<const T*>(param), g, h2[0], h2[1],
-                          h2[2], power_of_two_inverse(h2[0]), power_of_two_inverse(h2[1]), power_of_two_inverse(h2[2]),
+                          h2[2], exact_inverse(h2[0]), exact_inverse(h2[1]), exact_inverse(h2[2]),
                           chunks);
     });
     return AFSI_OK;

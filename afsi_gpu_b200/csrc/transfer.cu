@@ -265,14 +265,6 @@ extern "C" int32_t afsi_b200_indexed_spread(const void* field, int64_t points, i
 
 namespace {
 
-// 1/v when multiplying by it rounds as the division does (v a power of two), else 0.
-template <class T>
-T exact_inverse(T v) {
-    int ex = 0;
-    const T inv = T(1) / v;
-    return std::frexp(double(v), &ex) == 0.5 && std::isnormal(inv) && std::isnormal(v) ? inv : T(0);
-}
-
 template <class T, bool Spread>
 int32_t launch_compact(const CompactArgs<T>& a, int components, double volume, int32_t* status, cudaStream_t stream) {
     const dim3 grid(blocks_for(a.points * 4, 256), unsigned(components));
