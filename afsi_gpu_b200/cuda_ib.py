@@ -164,24 +164,25 @@ def _component_tables(grid, values, stencil, like):
 # The binned spread wins where many points share a cell.  What it saves grows with
 # the points and with how many share one; what it costs is a fixed 30 us of binning
 # and, per cell of the grid, two words that are cleared and scanned.  One B200, points
-# per occupied cell from which it is the faster form (a shell's cloud in any order,
+# per occupied cell from which it is the faster form (a thin shell's cloud in any order,
 # both spreads with all their launches and scratch), FP64: 60,000 points 20 on 64^3 and
 # 30 on 128^3; 100,000 14 and 20; 200,000 below 12 and 14; 256^3 50 at 200,000, 15 at
 # 400,000, 4 at a million; 512^3 none up to a million (60,000: 840 against 490 us and
 # 1.1 GB of scratch).  In FP32 the plain form's reductions cost less and the sums on
-# chip have no tensor cores: 60,000 points 50 on 64^3 and none on 128^3; 100,000 40;
-# 200,000 22 on 64^3, 25 on 128^3, 38 on 192^3; more points 16 to 22 up to 192^3; 256^3
-# none at any.  How many share a cell is sampled once, when the points are binned
-# (bin_density_kernel), and read with the support flag; the sample counts by points, so a
-# cloud whose cells are unevenly full reads denser than its mean, this shell by a third.
-# With the lines below, over 618 clouds of 9 to 64 per cell on 32^3 to 256^3, the form
-# taken is 0.5 % slower than the faster one on average, where 12 per cell for every type
-# and grid was 7.7 % slower.
+# chip have no tensor cores: 60,000 points 20 on 32^3, 50 on 64^3 and none on 128^3;
+# 100,000 40; 200,000 22 on 64^3, 25 on 128^3, 38 on 192^3; more points 16 to 22 up to
+# 192^3; 256^3 none at any.  How many share a cell is sampled once, when the points are
+# binned (bin_density_kernel), and read with the support flag; the sample counts by
+# points, so a cloud whose cells are unevenly full reads denser than its mean, a thin
+# shell by a third.  With the lines below, over 748 clouds of each type, thin and thick,
+# 3 to 96 per cell, 60,000 to a million points on 32^3 to 256^3, the form taken is 0.5 %
+# (FP64) and 0.7 % (FP32) slower than the faster one on average, where 12 per cell on
+# every grid was 2.7 and 10.7 % slower.
 _BINNED_POINTS = 60000
 # points at which `even` per cell break even: on the smallest grid, more up to 64^3 cells (FP32, where the plain
 # form's reductions meet less), and a fiftieth of the cells; even (in proportion to the points), the least per cell,
 # the most cells per point, the most cells
-_BINNED = {torch.float64: (64000, 0, 20., 12., 96, 1 << 62), torch.float32: (60000, 44000, 40., 26., 40, 1 << 23)}
+_BINNED = {torch.float64: (64000, 0, 16., 9., 96, 1 << 62), torch.float32: (40000, 60000, 32., 22., 40, 1 << 23)}
 
 
 def _binned_per_cell(points, shape, dtype):
