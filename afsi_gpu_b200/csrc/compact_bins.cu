@@ -15,7 +15,7 @@
 // directly.
 //
 // What bounds it is latency at 20 warps per SM (96 registers, 9.5 KB of shared
-// memory a warp), first of all the scattered reads of the table rows.  Lanes
+// memory a warp; issue 47 %), first of all the scattered reads of the table rows.  Lanes
 // therefore read whole rows together (cp.async, 16 bytes each), the bases and
 // forces of all components are requested at once, and the next component's rows
 // are in flight while a box is flushed: 186 -> 138 us; 32 points per warp at 20

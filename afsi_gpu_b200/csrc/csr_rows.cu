@@ -27,14 +27,14 @@
 //              radix sort on the face index alone (32-bit keys and positions).
 //
 // No atomics on values: the operators are the same bit for bit on every run.
-// What bounds it: the fill is bound by shared memory (64 links per point and
-// component, each cell visited by its four nodes; adding every point by itself
-// kept the shared-memory pipe 80 % busy), the finish by the HBM passes of the
-// sort.  128,000 tetrahedra (1.2 M points) on 128^3, FP64, one B200: fill
-// 0.80 ms (1.04 ms point by point), sorts 0.39 ms, pack and transpose 0.29 ms
+// What bounds it: the fill is bound by the L1's data stage (73 %; 64 links per
+// point and component added in shared memory, each cell visited by its four nodes;
+// adding every point by itself kept it 80 % busy), the finish by the HBM passes of
+// the sort.  128,000 tetrahedra (1.2 M points) on 128^3, FP64, one B200: fill
+// 0.78 ms (1.04 ms point by point), sorts 0.39 ms, pack and transpose 0.29 ms
 // for the three components, where the hash contraction took 4.98 ms and the
 // table's sorts 2.57 ms; tables, assembly, spread and interpolate together
-// 9.64 -> 2.39 ms.
+// 9.64 -> 2.38 ms.
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
 #include <algorithm>

@@ -33,7 +33,7 @@
 // and sums one point per lane over it.
 //
 // Bound by instruction issue and dependent latency at 16 warps per SM (56 % and
-// 49 % active).  38,400 P2 elements of 64 points on 64^3, FP64, one B200: spread
+// 50 % active; the L1's data stage 62 % and 75 %).  38,400 P2 elements of 64 points on 64^3, FP64, one B200: spread
 // 433 -> 403 us and gather 295 -> 280 us with each basis row read once and by
 // pairs (the rows of a warp's points touch a sector per lane: 101 M sectors and an
 // L1 71 % busy before), the force factors of the three components formed
@@ -835,7 +835,7 @@ __global__ void __launch_bounds__(kGWarps * 32, 4) fused_gather_kernel(
 // reads axis a on lattice a != c: from 0 to 1 axes 0 and 1, from 1 to 2 axes 1
 // and 2), so the third is kept: 7 rows per point instead of 9, the same values.
 
-// Bound by instruction issue (64 % and 67 % active at 16 and 24 warps per SM).
+// Bound by instruction issue (59 % and 67 % active at 16 and 24 warps per SM).
 // 128,000 P1 elements of 8 and 15 points on 128^3, FP32 beside FP64 positions,
 // one B200: spread 677 -> 233 us (345 us with one box copy and a point per
 // warp step instead of a point per half-warp), gather-assemble 442 -> 126 us.

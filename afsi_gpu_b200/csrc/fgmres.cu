@@ -211,12 +211,13 @@ __global__ void __launch_bounds__(kT) precondition_result_kernel(const T* __rest
 // kernel; w'' = w' - V^T c' with its norm; the scaled row.  Each kernel leaves
 // one partial per block, and every block of the next sums them in the same
 // fixed order (warp i takes the i-th sum), so nothing waits for a last block.
-// The passes are bound by reading V (L2 or HBM): 2 k n values for the two
-// projections of a step, against as many again for the separate matrix-vector
-// products, copies and norms they replace.  64^3 (1.06 M values), up to seven
-// rows, FP64, one B200: a coupled solve of six steps went from 6.78 to 5.15 ms
-// with these steps, the marching Helmholtz sweeps and the multigrid solve read
-// together with the step's column.
+// The passes read V four times (two projections and their dot products), as the
+// matrix-vector products did that they replace; saved are launches, copies of w
+// and of the column, and the norms' passes.  At 64^3 (1.06 M values) the
+// vectors stay in the L2 and latency bounds them: 9, 17, 14 and 9 us for two rows, the
+// L2 at 12 to 16 % of its rate.  Up to seven rows, FP64, one B200: a coupled solve of
+// six steps went from 6.78 to 5.15 ms with these steps, the marching Helmholtz sweeps
+// and the multigrid solve read together with the step's column.
 
 constexpr int kOrthoBlocks = 148 * 4;
 constexpr int kOrthoMost = 1024;  // basis rows

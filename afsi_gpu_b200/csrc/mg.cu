@@ -166,7 +166,10 @@ __device__ __forceinline__ void pair_neg_lap(const ZPair<T>& c, const ZPair<T>& 
 // owns the column of z pairs (y, z = 2k and 2k+1; nz even) and marches
 // `planes` planes along x, keeping the pair before, at and after the plane in
 // registers, so p is read from the L2 once and not three times (a plane per
-// thread read 89 MB per sweep at 128^3, 14 us; now 57 MB, 12 us).  The pair's
+// thread read 89 MB per sweep at 128^3, now 57 MB).  Bound by instruction issue and
+// dependent latency: 128^3, FP64, one B200, 13.5 us alone and about 10 in a solve,
+// 66 % of the issue slots, FP64 pipe 32 %, L2 19 %; a solve of twelve cycles 3.09 ->
+// 2.74 ms with the octet prolongation and the pending means.  The pair's
 // values and its y neighbours are 16-byte loads, the outer z neighbours two
 // scalars.  No pending shift of p (the launched sweeps take none); fix_rhs
 // subtracts the rhs mean and writes it back.  Per cell the same operations in
@@ -1837,8 +1840,9 @@ extern "C" int32_t afsi_b200_mg_residual_norm_noalloc(const void* p, const void*
 // block copies its map word and instance entry, the omega/diag table included,
 // to shared memory before it waits for the preceding operation: they are
 // constant, and their loads are two dependent round trips.  A step of 60
-// instances (FP64 tolerance, ten cycles, one B200) takes 2110 us instead of
-// 2555 with rows eight apart and the entries read after the wait.
+// instances (FP64 tolerance, ten cycles, one B200) went from 2555 us, with rows
+// eight apart and the entries read after the wait, to 2110; 61 us of that are the
+// spread's (batch_spread2d_kernel) and 50 the coarse blocks' (block_smooth).
 
 namespace afsi {
 

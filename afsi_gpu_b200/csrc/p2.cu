@@ -23,10 +23,12 @@
 // Rules of at most 64 points per element take a spread variant that stages the
 // element's stencil rows in shared memory with bulk copies first and merges
 // the points with the same support origin before adding them to a single box
-// copy (p2_spread_rows_kernel, runs.cuh).  12 warps per SM bound it (20 KB of
-// shared memory each); 38,400 elements of 64 points, FP64, one B200: 488 -> 479 us
-// with the basis rows read once, the groups placed by a scan and the boxes reduced
-// by redux (the gather 311 -> 301).  Rows kept from one component to the next made
+// copy (p2_spread_rows_kernel, runs.cuh).  10 warps per SM bound it (42 KB of
+// shared memory for two; issue 37 %); 38,400 elements of 64 points, FP64, one B200:
+// 488 -> 479 us with the basis rows read once, the groups placed by a scan and the
+// boxes reduced by redux.  The gather, 311 -> 301, is bound by the L1's data stage
+// (92 %); a whole pass of prepare, spread and gather shows no more than its runs
+// differ by.  Rows kept from one component to the next made
 // the gather slower (342 us: bound by the shared-memory pipe).
 // Point forces F = (Σ_a N[q,a] value[a]) * W (mac/compact_transfer.py:29-35)
 // are computed once per point and component by a lanes-over-points pass; the

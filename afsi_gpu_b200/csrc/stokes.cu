@@ -109,10 +109,11 @@ __global__ void __launch_bounds__(256) helmholtz_initialize_kernel(ConstFaces<T>
 }
 
 // One sweep.  ih2[a]: 1/h_a^2 where h_a^2 is a power of two (the product then
-// rounds as the quotient does), else 0.  Bound by the L2 (u, rhs, diag in, u
-// out, 26 MB at 64^3) and, at 64^3, by the launch: 12.8 us with a thread per
-// face and three 64-bit divisions for its coordinates, 9.7 us with the
-// marching columns and programmatic dependent launch.
+// rounds as the quotient does), else 0.  Bound by instruction issue (68 % of
+// the slots at 64^3; a division by the diagonal per face; the L2, u, rhs, diag in and
+// u out, at 12 %): 64^3, FP64, one B200, 12.8 us with a thread per face and three
+// 64-bit divisions for its coordinates, 9.7 us with the marching columns and
+// programmatic dependent launch.
 template <class T>
 __global__ void __launch_bounds__(256) helmholtz_sweep_kernel(ConstFaces<T> u, ConstFaces<T> rhs, ConstFaces<T> diag,
                                                               Faces<T> out, const T* __restrict__ param, Cells g,

@@ -313,8 +313,10 @@ int32_t afsi_b200_compact_spread3(const void* force, const int64_t* base, const 
  * cell or tile are summed on chip and reduced into a face once.  Same
  * arguments; phi 16-byte aligned, points < 2^31 - 1, and `scratch` of at least
  * compact_binned_bytes (-1: sizes that only spread3 takes).  */
-/* compact_density sets `bit` of the status word when the points, by a sample,
- * hold more than per_cell of them per occupied cell of component 0's base. */
+/* compact_density sets `bit` of the word at `status` when the points, by a
+ * sample, hold more than per_cell of them per occupied cell of component 0's
+ * base: a word of the question's own, as readers of a shared one take any bit
+ * for a violation. */
 int32_t afsi_b200_compact_density(const int64_t* base, int64_t points, double per_cell, int32_t bit,
     int32_t* status, afsi_stream_t stream);
 int64_t afsi_b200_compact_binned_bytes(int64_t points, int64_t nx, int64_t ny, int64_t nz);
