@@ -13,6 +13,7 @@ Beyond the reference operators this module exposes the binning kernels
 (:func:`compact_prepare`, :func:`prepare2d`), which the reference runs as torch
 expressions.
 """
+import threading
 from dataclasses import dataclass
 from math import prod
 import torch
@@ -267,6 +268,24 @@ class CompactStencil:
         return CompactStencil(base, phi, 'component')
 
 
+_ROWS = 256
+_rows, _rows_lock = {}, threading.Lock()
+
+
+def _own_words(device):
+    """Two zeroed int32 words of one call's own, read by the host before the call
+    returns: rows of a block per device, each given out once.  The block is cleared
+    and waited for when it is made, so its rows serve every stream (a fill per call
+    cost 3 us of the 165 that 84,000 points on 32 x 32 x 16 take)."""
+    with _rows_lock:
+        block, given = _rows.get(device.index, (None, _ROWS))
+        if given == _ROWS:
+            block, given = torch.zeros((_ROWS, 2), device=device, dtype=torch.int32), 0
+            torch.cuda.current_stream(device).synchronize()
+        _rows[device.index] = block, given + 1
+    return block[given]
+
+
 def compact_prepare(grid, points, *, layout='component', phi_form='clamped', check_support=True):
     """Binning + weights of ``mac/compact_transfer.py:21-26`` (``from_points``),
     with the support screen of ``compact_transfer.py:94-96`` fused.
@@ -295,7 +314,7 @@ def compact_prepare(grid, points, *, layout='component', phi_form='clamped', che
     per_cell = _binned_per_cell(P, grid.shape, points.dtype) if check_support and layout == 'component' else None
     ask = per_cell is not None
     if ask:
-        own = torch.zeros(2, device=points.device, dtype=torch.int32)
+        own = _own_words(points.device)
     else:
         own = word.zero_() if check_support else word
     call('afsi_b200_compact_prepare', ptr(points), P, L, _lib.doubles(sum(map(list, origins), [])),

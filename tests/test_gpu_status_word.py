@@ -55,3 +55,22 @@ def test_a_dense_cloud_keeps_the_flags_of_others(monkeypatch):
     with pytest.raises(ValueError, match='support'):
         cuda_ib.compact_prepare(grid, x)
     assert cuda_ib.check() == 0
+
+
+def test_no_pair_of_words_is_given_out_twice():
+    """Rows of used-up blocks are not zeroed again: every call gets a fresh one, on every stream."""
+    grid, x = _dense()
+    streams = [torch.cuda.current_stream(), torch.cuda.Stream(), torch.cuda.Stream()]
+    held = [cuda_ib._own_words(x.device) for _ in range(2 * cuda_ib._ROWS)]
+    assert len({w.data_ptr() for w in held}) == len(held) and not any(bool(w.any()) for w in held)
+    sparse = .1 + .8 * torch.rand((70000, 3), device=DEV, dtype=torch.float64)
+    bad = x.clone()
+    bad[3, 1] = float('nan')
+    torch.cuda.synchronize()
+    for k in range(cuda_ib._ROWS + 10):
+        with torch.cuda.stream(streams[k % 3]):
+            if k % 50 == 7:
+                with pytest.raises(ValueError, match='support'):
+                    cuda_ib.compact_prepare(grid, bad)
+            else:
+                assert cuda_ib.compact_prepare(grid, x if k % 2 else sparse).dense == bool(k % 2)
